@@ -156,6 +156,10 @@ PMArgs make_args(hpm_ctx *c)
     a.cand_costs = c->d_cand;
     a.cand_pos = c->d_pos;
     a.cand_flags = c->d_flags;
+    const size_t nh = ((size_t)a.W * a.H + 1) / 2;
+    a.rf_plane = c->d_refine;
+    a.rf_state = c->d_refine + nh;
+    a.rf_views = reinterpret_cast<uint32_t *>(c->d_refine + 2 * nh);
     a.proposals = c->proposals;
     a.geom_max = 5.0f; /* HPM.cu:485 */
     return a;
@@ -250,6 +254,7 @@ int hpm_destroy(hpm_ctx *c)
     cudaFree(c->d_cand);
     cudaFree(c->d_pos);
     cudaFree(c->d_flags);
+    cudaFree(c->d_refine);
     cudaFree(c->d_pre);
     ws_free(c);
     net_free(c);
@@ -321,6 +326,7 @@ int hpm_set_views(hpm_ctx *c, const float *const *images, const HpmCamera *cams,
     CK(ensure((void **)&c->d_cand, &c->cand_cap, sizeof(float) * nh * (num_images - 1) * kCandRows), "cand alloc");
     CK(ensure((void **)&c->d_pos, &c->pos_cap, sizeof(int) * nh * 8), "cand alloc");
     CK(ensure((void **)&c->d_flags, &c->flags_cap, sizeof(uint32_t) * nh), "cand alloc");
+    CK(ensure((void **)&c->d_refine, &c->refine_cap, sizeof(float4) * nh * 3), "cand alloc");
     CK(cudaMemsetAsync(c->d_planes, 0, sizeof(float4) * n, c->stream), "state clear");
     CK(cudaMemsetAsync(c->d_costs, 0, sizeof(float) * n, c->stream), "state clear");
     CK(cudaMemsetAsync(c->d_views, 0, sizeof(uint32_t) * n, c->stream), "state clear");

@@ -113,6 +113,8 @@ struct hpm_ctx {
     size_t pos_cap = 0;
     uint32_t *d_flags = nullptr; /* direction row codes [ceil(H*W/2)] */
     size_t flags_cap = 0;
+    float4 *d_refine = nullptr; /* selection to refinement: plane, state and view weights [3][ceil(H*W/2)] */
+    size_t refine_cap = 0;
     float *d_pre = nullptr; /* ACMM+NESP hierarchy pass: acceptance threshold per pixel */
     size_t pre_cap = 0;
 

@@ -65,6 +65,12 @@ struct PMArgs {
     float *cand_costs;
     int *cand_pos;
     uint32_t *cand_flags;
+    /* hand-off from the selection to the refinement, per slot: the plane after
+     * the neighbours, (cost, depth, restricted cost, current cost), and the
+     * view weights, 4 bits per view (2 words up to 16 sources, else 4) */
+    float4 *rf_plane;
+    float4 *rf_state;
+    uint32_t *rf_views;
     unsigned long long *counters; /* [2]: cost vectors, geom terms, or nullptr */
     /* prior-net form: per pixel a proposed plane (ref-frame normal, distance),
      * scored as one more refinement candidate; nullptr in the plain form */

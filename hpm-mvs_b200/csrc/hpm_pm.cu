@@ -9,21 +9,20 @@
  *    weights of a pixel's 11x11/stride-2 window (one exp, one sqrt, two
  *    divides each) and all reference-side sums inside every NCC call
  *    (HPM.cu:345-368), i.e. ~23 x S times per pixel per half-step.  Here they
- *    are computed once per pixel per launch, with the reference's own
- *    expressions (so the values are the same bits), and kept in shared memory
- *    as a [tap][thread] array: each NCC tap then costs one shared load of the
- *    weight and one of weight*ref instead of an exp, a sqrt and two texture
- *    fetches.
+ *    are computed once per pixel per launch and kept in shared memory, beside
+ *    a tile of the reference image: each NCC tap then costs shared loads
+ *    instead of an exp, a sqrt and two texture fetches.
  *  - Source views are sampled by the texture unit (float cudaArray, linear
  *    filter, clamped edges: the reference's own texture set-up), so the
  *    bilinear samples are the reference's bit for bit.  The filter rounds
  *    coordinates to 1/256 (half up) and only the far corner's weight
  *    A*B/256; a textbook bilinear gather differs by up to ~0.5 gray levels
  *    per tap.
+ *  - A warp scores its pixels' windows together (ncc_quad), packed 32 at a
+ *    time whatever pixel they belong to.
  *  - The per-pixel cost matrix (cost_array[8][32], 1.5 KB of local memory per
  *    thread in the reference) is handed from the site/direction kernel to the
- *    selection/refinement kernel through L2, so that shared memory holds only
- *    the 288-byte reference window per pixel.
+ *    selection and the refinement through L2.
  *  - Counter-based Philox random numbers: no 48-byte curand state per pixel
  *    in HBM and no curand_init skip-ahead; draws come in the reference's
  *    order.
@@ -60,14 +59,17 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
     px = bx * (2 * ww) + 2 * (lane % ww) + ((py + color) & 1);
 }
 
-#ifndef HPM_CV_INLINE
-#define HPM_CV_INLINE __noinline__
-#endif
+/* Blocks per SM that the window kernels are compiled for.  At 7 (14 warps,
+ * 144 registers) nothing spills and the blocks' shared memory leaves 92 KB or
+ * more to the texture cache; 10 and 6 blocks are slower (k_prop_dirs at
+ * 1600x1200 with 10 sources: 3.41 and 3.77 against 3.42 ms, at 641x481 with 4:
+ * 0.318 and 0.327 against 0.300; k_prop_refine 1.60 against 1.57 and 0.161
+ * against 0.151). */
 #ifndef HPM_P1_MIN_BLOCKS
-#define HPM_P1_MIN_BLOCKS 10
+#define HPM_P1_MIN_BLOCKS 7
 #endif
 #ifndef HPM_P2_MIN_BLOCKS
-#define HPM_P2_MIN_BLOCKS 10
+#define HPM_P2_MIN_BLOCKS 7
 #endif
 
 /* ------------------------------------------------------------------ */
@@ -110,6 +112,14 @@ struct Rng {
         b3 = c3;
     }
 
+    /* the stream after `drawn` draws */
+    __device__ void resume(uint32_t klo, uint32_t khi, uint32_t px, uint32_t st, uint32_t sa, uint32_t drawn)
+    {
+        init(klo, khi, px, st, sa);
+        n = drawn;
+        if (n & 3u) block();
+    }
+
     /* uniform in (0,1]: ((x >> 8) + 1) * 2^-24 */
     __device__ float uniform()
     {
@@ -133,14 +143,153 @@ __device__ __forceinline__ float texel(const float *__restrict__ img, int w, int
     return __ldg(img + (size_t)y * w + x);
 }
 
-/* The hoisted reference window has one entry per tap and pixel in shared
- * memory: (weight, weight x reference pixel) as float2 (WinPair), or the
- * weight alone (WinWeight), the reference pixel then being re-read through
- * L1 at each use.  The weight-only form halves the shared memory; it suits
- * k_init (2.75 against 4.7 ms at 1600x1200), while in the half-step kernels
- * the extra L1 loads compete with the texture path (10.2 against 5.4 ms). */
-typedef float2 WinPair;
-typedef float WinWeight;
+/* Two FP32 operations per instruction (fma/mul/add.f32x2): half the issue
+ * slots, each half rounded as the scalar operation. */
+__device__ __forceinline__ unsigned long long pack2(float2 a)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long r)
+{
+    float2 a;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+    return a;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    unsigned long long r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)), "l"(pack2(c)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    unsigned long long r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+/* The bilateral weight of a tap (HPM.cu:339-341) is exp(spatial + range):
+ * the spatial terms of the window's 6 x 6 taps depend on |i| and |j| only and
+ * are kept per block, those of rows 2 pair and 2 pair + 1 side by side. */
+struct Spatial {
+    float2 term[3][3]; /* [row pair][|j| = 5, 3, 1] */
+};
+
+__device__ __forceinline__ float rcp_approx(float a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+__device__ __forceinline__ void spatial_terms(float sigma, Spatial *out)
+{
+    const int t = threadIdx.y * kBlockX + threadIdx.x;
+    if (t < 18) {
+        const int i = 2 * (t / 3) - 5, j = 5 - 2 * (t % 3);
+        const float x = (float)i, y = (float)j;
+        const float term = -sqrtf(x * x + y * y) * rcp_approx(2.0f * sigma * sigma);
+        reinterpret_cast<float *>(&out->term[t / 6][t % 3])[(t / 3) & 1] = term;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ float tap_weight(float spatial, float ref, float center, float range_scale)
+{
+    return expf(__fmaf_rn(-fabsf(ref - center), range_scale, spatial));
+}
+
+/* The reference window of a pixel: its weights in shared memory, written once
+ * by ref_window ([row pair][column][thread]: the weights of two rows side by
+ * side for the packed sums of ncc_quad), and its pixels, read at each use from
+ * global memory (WinImage) or from a tile of the block's surroundings in
+ * shared memory (WinTile).  Computing the weights again at each use would
+ * halve the block's shared memory but costs more than the texture cache gains
+ * (refinement at 1600x1200, 10 sources: 1.80 against 1.57 ms). */
+struct WinImage {
+    const Spatial *sp;
+    float range_scale, mid;
+    float2 *w; /* this thread's column */
+    const float *img;
+    int W, H, px, py;
+    __device__ __forceinline__ float ref(int ti, int tj) const { return texel(img, W, H, px + 2 * ti - 5, py + 2 * tj - 5); }
+};
+
+/* Half-step blocks: every tap of a pixel has the pixel's own checkerboard
+ * colour (both offsets are odd), so the tile holds that colour only: row R is
+ * image row y = y0 - 5 + R, entry c of it the column
+ * x0 + par(y + 1) - 5 + 2 c, where par(y) = (y + colour) & 1 is the
+ * parity of the updated columns of row y.  A tap of the pixel at (lx, ly) of
+ * the block's patch is then row ly + 2 tj, entry lx + ti.  The pitch keeps a
+ * warp's rows (of WW pixels each) on different banks. */
+template <int WW>
+struct WinTile {
+    static constexpr int WH = 32 / WW, kRows = 2 * WH + 10, kCols = WW + 5;
+    static constexpr int kPitch = WW == 4 ? 12 : (WW == 8 ? 24 : 48);
+    const Spatial *sp;
+    float range_scale, mid; /* the pixel's own value */
+    float2 *w;              /* its column of weights */
+    const float *tile;      /* its first tap */
+    __device__ __forceinline__ float ref(int ti, int tj) const { return tile[2 * tj * kPitch + ti]; }
+};
+
+/* weights of rows 2 pair and 2 pair + 1 in column tj, given their pixels */
+template <typename Win>
+__device__ __forceinline__ float2 tap_weights(const Win &win, int pair, int tj, float2 ref)
+{
+    const float2 s = win.sp->term[pair][tj < 3 ? tj : 5 - tj];
+    return make_float2(tap_weight(s.x, ref.x, win.mid, win.range_scale), tap_weight(s.y, ref.y, win.mid, win.range_scale));
+}
+
+/* Shared memory of a half-step block and its place in the image.  Pixel q of
+ * the block (0 .. 63, a warp's 32 in lane order) lies at (x(q), y(q)). */
+template <int WW>
+struct Patch {
+    using Tile = WinTile<WW>;
+    const Spatial *sp;
+    float2 *w;
+    float *tile;
+    float range_scale;
+    int x0, y0, color;
+
+    __device__ __forceinline__ int y(int q) const { return y0 + q / WW; }
+    __device__ __forceinline__ int x(int q) const { return x0 + 2 * (q % WW) + ((y(q) + color) & 1); }
+    __device__ __forceinline__ Tile win(int q) const
+    {
+        const float *first = tile + q / WW * Tile::kPitch + q % WW;
+        return {sp, range_scale, first[5 * Tile::kPitch + 2 + ((y(q) + color) & 1)], w + q, first};
+    }
+};
+
+/* Shared memory of a half-step block's reference windows. */
+template <int WW>
+struct PatchMem {
+    using Tile = WinTile<WW>;
+    float2 w[kTaps / 2 * kBlock];
+    float tile[Tile::kRows * Tile::kPitch];
+    Spatial sp;
+
+    /* fills the tile (all threads; edges repeated) and the spatial terms */
+    __device__ __forceinline__ Patch<WW> load(const PMArgs &a, int color)
+    {
+        const ViewDev &rv = a.view[0];
+        const int x0 = (int)blockIdx.x * 2 * WW, y0 = (int)blockIdx.y * 2 * (32 / WW);
+        for (int i = threadIdx.y * kBlockX + threadIdx.x; i < Tile::kRows * Tile::kCols; i += kBlock) {
+            const int r = i / Tile::kCols, c = i - r * Tile::kCols, ty = y0 - 5 + r;
+            tile[r * Tile::kPitch + c] = texel(rv.img, rv.w, rv.h, x0 + ((ty + 1 + color) & 1) - 5 + 2 * c, ty);
+        }
+        spatial_terms(a.sigma_spatial, &sp);
+        return {&sp, w, tile, rcp_approx(2.0f * a.sigma_color * a.sigma_color), x0, y0, color};
+    }
+};
 
 /* ------------------------------------------------------------------ */
 /* Geometry (HPM.cu:65-133, 227-316, 445-481)                           */
@@ -291,127 +440,201 @@ __device__ __forceinline__ float2 warp(const float *H, float px, float py)
 /* Hoisted reference window                                            */
 /* ------------------------------------------------------------------ */
 
+__device__ __forceinline__ WinImage image_window(const PMArgs &a, const Spatial *sp, float2 *w, int px, int py)
+{
+    return {sp, rcp_approx(2.0f * a.sigma_color * a.sigma_color), texel(a.view[0].img, a.W, a.H, px, py), w,
+            a.view[0].img, a.W, a.H, px, py};
+}
+
 struct RefStats {
     float inv;  /* 1 / sum of weights */
     float mean; /* weighted mean of the reference window */
     float var;  /* weighted variance of the reference window */
 };
 
-/* The reference-side half of ComputeBilateralNCC (HPM.cu:318-386) for pixel
- * (px, py): per-tap (weight, weight*ref) into shared memory as one float2,
- * sums in the reference's row-then-total order.  sWW is [tap][kBlock]. */
+/* The reference-side half of ComputeBilateralNCC (HPM.cu:318-386) of a
+ * thread's pixel: per-tap weights into shared memory, sums in the reference's
+ * row-then-total order. */
 template <typename Win>
-__device__ RefStats ref_window(const PMArgs &a, int px, int py, Win *sWW, int tid)
+__device__ RefStats ref_window(const Win &win)
 {
-    const ViewDev &rv = a.view[0];
-    const float center = texel(rv.img, rv.w, rv.h, px, py);
     float sum_ref = 0.0f, sum_ref_ref = 0.0f, wsum = 0.0f;
-    int t = 0;
-    for (int i = -5; i < 6; i += 2) {
-        float r_ref = 0.0f, r_rr = 0.0f, r_w = 0.0f;
-        for (int j = -5; j < 6; j += 2, ++t) {
-            const float rp = texel(rv.img, rv.w, rv.h, px + i, py + j);
-            const float x_dist = (float)i, y_dist = (float)j;
-            const float spatial_dist = sqrtf(x_dist * x_dist + y_dist * y_dist);
-            const float color_dist = fabsf(rp - center);
-            const float wgt = expf(-spatial_dist / (2.0f * a.sigma_spatial * a.sigma_spatial) -
-                                   color_dist / (2.0f * a.sigma_color * a.sigma_color));
-            if constexpr (sizeof(Win) == sizeof(float))
-                sWW[t * kBlock + tid] = wgt;
-            else
-                sWW[t * kBlock + tid] = make_float2(wgt, wgt * rp);
-            r_ref += wgt * rp;
-            r_rr += wgt * rp * rp;
-            r_w += wgt;
+    for (int pair = 0; pair < 3; ++pair) {
+        float2 r_ref = make_float2(0.0f, 0.0f), r_rr = r_ref, r_w = r_ref;
+#pragma unroll
+        for (int tj = 0; tj < 6; ++tj) {
+            const float2 rp = make_float2(win.ref(2 * pair, tj), win.ref(2 * pair + 1, tj));
+            const float2 wgt = tap_weights(win, pair, tj, rp);
+            win.w[(pair * 6 + tj) * kBlock] = wgt;
+            const float2 m = mul2(wgt, rp);
+            r_ref = add2(r_ref, m);
+            r_rr = fma2(m, rp, r_rr);
+            r_w = add2(r_w, wgt);
         }
-        sum_ref += r_ref;
-        sum_ref_ref += r_rr;
-        wsum += r_w;
+        sum_ref = __fadd_rn(__fadd_rn(sum_ref, r_ref.x), r_ref.y);
+        sum_ref_ref = __fadd_rn(__fadd_rn(sum_ref_ref, r_rr.x), r_rr.y);
+        wsum = __fadd_rn(__fadd_rn(wsum, r_w.x), r_w.y);
     }
     RefStats s;
     s.inv = 1.0f / wsum;
     s.mean = sum_ref * s.inv;
-    const float mrr = sum_ref_ref * s.inv;
-    s.var = mrr - s.mean * s.mean;
+    s.var = __fmaf_rn(sum_ref_ref, s.inv, -__fmul_rn(s.mean, s.mean));
     return s;
 }
 
-/* Source sample of tap (i, j) of pixel (fpx, fpy): the warped tap position
- * (ComputeCorrespondingPoint, HPM.cu:289-296) through the texture unit at
- * +0.5 (HPM.cu:358-359).  One definition for the NCC and the tap-sample
- * export, so that both evaluate the same expression. */
-__device__ __forceinline__ float tap_sample(cudaTextureObject_t tex, const float *H, float fpx, float fpy, int i, int j)
+/* Nine source samples of a window, one of each 2 x 2 block of its taps: at
+ * (x0 + 4 bi, y0 + 4 bj), the warped position (ComputeCorrespondingPoint,
+ * HPM.cu:289-296) through the texture unit at +0.5 (HPM.cu:358-359).  One
+ * definition for the NCC and the tap-sample export, so that both evaluate the
+ * same expression. */
+__device__ __forceinline__ void fetch_block(cudaTextureObject_t tex, const float *H, float x0, float y0, float *s)
 {
-    const float2 q = warp(H, fpx + (float)i, fpy + (float)j);
-    return tex2D<float>(tex, q.x + 0.5f, q.y + 0.5f);
+    const float2 Hx = make_float2(H[0], H[3]), Hy = make_float2(H[1], H[4]), Hc = make_float2(H[2], H[5]);
+    float2 my[3];
+    float mz[3];
+#pragma unroll
+    for (int bj = 0; bj < 3; ++bj) {
+        const float y = y0 + (float)(4 * bj);
+        my[bj] = mul2(Hy, both(y));
+        mz[bj] = __fmul_rn(H[7], y);
+    }
+#pragma unroll
+    for (int bi = 0; bi < 3; ++bi) {
+        const float x = x0 + (float)(4 * bi);
+        const float2 z01 = add2(fma2(both(H[6]), both(x), make_float2(mz[0], mz[1])), both(H[8]));
+        const float z2 = __fadd_rn(__fmaf_rn(H[6], x, mz[2]), H[8]);
+#pragma unroll
+        for (int bj = 0; bj < 3; ++bj) {
+            const float2 xy = add2(fma2(Hx, both(x), my[bj]), Hc);
+            const float2 q = add2(mul2(xy, both(rcp_approx(bj == 0 ? z01.x : (bj == 1 ? z01.y : z2)))), both(0.5f));
+            s[bi * 3 + bj] = tex2D<float>(tex, q.x, q.y);
+        }
+    }
 }
 
-/* The source-side half of ComputeBilateralNCC (HPM.cu:325-397). */
-template <typename Win>
-__device__ __forceinline__ float ncc(const PMArgs &a, int v, int px, int py, float4 h, const Win *sWW, int tid,
-                                     const RefStats &rs)
+constexpr unsigned kAll = 0xffffffffu; /* a whole warp */
+
+/* a or b, by a byte selector (0x3210 or 0x7654) */
+__device__ __forceinline__ float pick(float a, float b, unsigned sel)
 {
+    return __uint_as_float(__byte_perm(__float_as_uint(a), __float_as_uint(b), sel));
+}
+
+/* The source-side half of ComputeBilateralNCC (HPM.cu:325-397), one window
+ * per lane, for the whole warp at once: every lane passes the pixel (px, py),
+ * plane, reference window and statistics of the window it wants, and whether
+ * it wants one (need); all 32 lanes must call, with the same view.
+ *
+ * The four lanes of a quad fetch one window at a time, a 2 x 2 block of its
+ * taps per texture instruction, then hand the samples to the window's own
+ * lane, which sums them in the reference's order.  The texture unit serves a
+ * quad whose taps lie together at 2.9 to 3.1 taps per clock and SM whatever
+ * the planes of neighbouring pixels; with one window per lane, as many taps of
+ * unrelated windows in a quad run at 1.2, and at 0.5 with little texture
+ * cache.  Products and sums are paired into two-wide instructions, since the
+ * issue slots are the next bound, with the roundings spelled out.
+ *
+ * The view goes through a shuffle so that the compiler takes it as the same
+ * in all lanes: otherwise each texture instruction becomes a loop over the
+ * distinct texture handles of its lanes (k_prop_refine at 1600x1200, 10
+ * sources: 3.70 against 1.80 ms). */
+template <typename Win>
+__device__ __forceinline__ float ncc_quad(const PMArgs &a, int v, int px, int py, bool need, float4 h, const Win &win,
+                                          const RefStats &rs)
+{
+    v = __shfl_sync(kAll, v, 0);
     const HpmCamera &sc = a.cam[v];
     float H[9];
     homography(a.cam[0], sc, a.pair[v], h, H);
     const float fpx = (float)px, fpy = (float)py;
     const float2 pt = warp(H, fpx, fpy);
-    if (pt.x >= sc.width || pt.x < 0.0f || pt.y >= sc.height || pt.y < 0.0f) return 2.0f;
-    if (rs.var < 1e-5f) return 2.0f; /* the reference reaches the same result after the taps */
+    /* the reference reaches 2 for a flat window after the taps */
+    const bool go = need && !(pt.x >= sc.width || pt.x < 0.0f || pt.y >= sc.height || pt.y < 0.0f) &&
+                    !(rs.var < 1e-5f);
+    const unsigned ball = __ballot_sync(kAll, go);
+    if (ball == 0) return 2.0f;
     const cudaTextureObject_t tex = a.view[v].tex;
-    float sum_src = 0.0f, sum_src_src = 0.0f, sum_ref_src = 0.0f;
-    int t = 0;
+    const int lane = threadIdx.x, l = lane & 3;
+    const unsigned quad = (ball >> (lane & 28)) & 15u;
+    float s[4][9];
 #pragma unroll
-    for (int i = -5; i < 6; i += 2) {
-        float r_src = 0.0f, r_ss = 0.0f, r_rs = 0.0f;
+    for (int w = 0; w < 4; ++w) {
+        float G[9];
 #pragma unroll
-        for (int j = -5; j < 6; j += 2, ++t) {
-            const float sp = tap_sample(tex, H, fpx, fpy, i, j);
-            float2 ww;
-            if constexpr (sizeof(Win) == sizeof(float)) {
-                const float wt = sWW[t * kBlock + tid];
-                ww = make_float2(wt, wt * texel(a.view[0].img, a.view[0].w, a.view[0].h, px + i, py + j));
-            } else {
-                ww = sWW[t * kBlock + tid];
-            }
-            r_src += ww.x * sp;
-            r_ss += ww.x * sp * sp;
-            r_rs += ww.y * sp;
+        for (int e = 0; e < 9; ++e) G[e] = __shfl_sync(kAll, H[e], w, 4);
+        const float gx = __shfl_sync(kAll, fpx, w, 4), gy = __shfl_sync(kAll, fpy, w, 4);
+#pragma unroll
+        for (int b = 0; b < 9; ++b) s[w][b] = 0.0f;
+        if ((quad >> w) & 1u) {
+            /* lane l takes tap l ^ w of each block (bit 0: along x, bit 1:
+             * along y), so that the hand-over below needs no select on the
+             * receiving side */
+            const int tp = l ^ w;
+            fetch_block(tex, G, gx + (float)(2 * (tp & 1) - 5), gy + (float)(2 * (tp >> 1) - 5), s[w]);
         }
-        sum_src += r_src;
-        sum_src_src += r_ss;
-        sum_ref_src += r_rs;
     }
-    sum_src *= rs.inv;
-    sum_src_src *= rs.inv;
-    sum_ref_src *= rs.inv;
-    const float var_src = sum_src_src - sum_src * sum_src;
-    if (var_src < 1e-5f) return 2.0f;
-    const float covar = sum_ref_src - rs.mean * sum_src;
+    /* byte selectors, not predicates: too many are live for those */
+    const unsigned pick1 = (l & 1) ? 0x7654u : 0x3210u, pick2 = (l & 2) ? 0x7654u : 0x3210u;
+    float sum_src = 0.0f, sum_src_src = 0.0f, sum_ref_src = 0.0f;
+#pragma unroll
+    for (int bi = 0; bi < 3; ++bi) {
+        /* rows 2 bi and 2 bi + 1 side by side */
+        float2 r_src = make_float2(0.0f, 0.0f), r_ss = r_src, r_rs = r_src;
+#pragma unroll
+        for (int bj = 0; bj < 3; ++bj) {
+            const int b = bi * 3 + bj;
+            /* p[d] = s[l ^ d][b]: what lane l ^ d is waiting for */
+            float q[4], p[4], tap[4];
+#pragma unroll
+            for (int d = 0; d < 4; ++d) q[d] = pick(s[d][b], s[d ^ 1][b], pick1);
+#pragma unroll
+            for (int d = 0; d < 4; ++d) p[d] = pick(q[d], q[d ^ 2], pick2);
+            tap[0] = p[0];
+#pragma unroll
+            for (int d = 1; d < 4; ++d) tap[d] = __shfl_xor_sync(kAll, p[d], d);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 sp = make_float2(tap[2 * e], tap[2 * e + 1]);
+                const float2 rp = make_float2(win.ref(2 * bi, 2 * bj + e), win.ref(2 * bi + 1, 2 * bj + e));
+                const float2 wt = win.w[(bi * 6 + 2 * bj + e) * kBlock], wr = mul2(wt, rp);
+                const float2 m = mul2(wt, sp);
+                r_src = add2(r_src, m);
+                r_ss = fma2(m, sp, r_ss);
+                r_rs = fma2(wr, sp, r_rs);
+            }
+        }
+        sum_src = __fadd_rn(__fadd_rn(sum_src, r_src.x), r_src.y);
+        sum_src_src = __fadd_rn(__fadd_rn(sum_src_src, r_ss.x), r_ss.y);
+        sum_ref_src = __fadd_rn(__fadd_rn(sum_ref_src, r_rs.x), r_rs.y);
+    }
+    const float mean_src = __fmul_rn(sum_src, rs.inv);
+    const float var_src = __fmaf_rn(sum_src_src, rs.inv, -__fmul_rn(mean_src, mean_src));
+    if (!go || var_src < 1e-5f) return 2.0f;
+    const float covar = __fmaf_rn(sum_ref_src, rs.inv, -__fmul_rn(rs.mean, mean_src));
     const float vv = sqrtf(rs.var * var_src);
     return fmaxf(0.0f, fminf(2.0f, 1.0f - covar / vv));
 }
 
-/* One NCC window for the loops that score several candidates view by view
- * (inline by default; -DHPM_NCC_CALL=__noinline__ builds it out of line). */
-#ifndef HPM_NCC_CALL
-#define HPM_NCC_CALL __forceinline__
-#endif
-template <typename Win>
-__device__ HPM_NCC_CALL float ncc_call(const PMArgs &a, int v, int px, int py, float4 h, const Win *sWW, int tid,
-                                        RefStats rs)
+/* another lane's statistics */
+__device__ __forceinline__ RefStats stats_of(const RefStats &rs, int lane)
 {
-    return ncc(a, v, px, py, h, sWW, tid, rs);
+    return {__shfl_sync(kAll, rs.inv, lane), __shfl_sync(kAll, rs.mean, lane), __shfl_sync(kAll, rs.var, lane)};
 }
 
-/* ComputeMultiViewCostVector (HPM.cu:438-443) into out[v * stride].  Kept
- * out of line so that the 36-tap loop exists once in the binary. */
+__device__ __forceinline__ unsigned lanes_below() { return (1u << threadIdx.x) - 1u; }
+
+/* ComputeMultiViewCostVector (HPM.cu:438-443) of the warp's pixels into
+ * out[v * stride] of the lanes that want it; all 32 lanes must call. */
 template <typename Win>
-__device__ HPM_CV_INLINE void cost_vector(const PMArgs &a, int px, int py, float4 h, const Win *sWW, int tid,
-                                         RefStats rs, float *out, int stride)
+__device__ __forceinline__ void cost_vector(const PMArgs &a, int px, int py, bool need, float4 h, const Win &win,
+                                            const RefStats &rs, float *out, int stride)
 {
-    for (int v = 1; v < a.n; ++v) out[(size_t)(v - 1) * stride] = ncc(a, v, px, py, h, sWW, tid, rs);
-    if (a.counters) atomicAdd(&a.counters[0], (unsigned long long)(a.n - 1));
+#pragma unroll 1
+    for (int v = 1; v < a.n; ++v) {
+        const float c = ncc_quad(a, v, px, py, need, h, win, rs);
+        if (need) out[(size_t)(v - 1) * stride] = c;
+    }
+    if (a.counters && need) atomicAdd(&a.counters[0], (unsigned long long)(a.n - 1));
 }
 
 __device__ __forceinline__ void sort_small(float *d, int n) /* HPM.cu:3-12 */
@@ -563,12 +786,15 @@ __device__ __forceinline__ float *cache_at(const PMArgs &a, int v, const Slot &s
 }
 
 /* RandomInitialization, HPM.cu:510-558.  One thread per pixel. */
-__device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, WinWeight *sWW, float *sCV, int tid)
+__device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, const Spatial &sp, float2 *sW, float *sCV, int tid)
 {
-    if (px >= a.W || py >= a.H) return;
-    const int center = py * a.W + px;
+    const bool act = px < a.W && py < a.H;
+    /* lanes outside the image stay for the warp's windows, on a pixel inside */
+    const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
+    const int center = cy * a.W + cx;
     const HpmCamera &cam = a.cam[0];
-    const RefStats rs = ref_window(a, px, py, sWW, tid);
+    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
+    const RefStats rs = ref_window(win);
     Rng rng;
     rng.init(a.seed_lo, a.seed_hi, (uint32_t)center, 0u, a.salt);
     float4 h;
@@ -582,15 +808,15 @@ __device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, WinWe
              * reference leaves it unset, taken as 0 */
             const float4 hz = make_float4(0.0f, 0.0f, 0.0f, a.planes[center].w);
             float *cvz = sCV + tid;
-            cost_vector(a, px, py, hz, sWW, tid, rs, cvz, kBlock);
+            cost_vector(a, px, py, act, hz, win, rs, cvz, kBlock);
             uint32_t unused;
-            a.pre_costs[center] = initial_cost_from(a, cvz, kBlock, &unused);
+            if (act) a.pre_costs[center] = initial_cost_from(a, cvz, kBlock, &unused);
         } else if (a.hier == 2) {
-            a.pre_costs[center] = 0.0f;
+            if (act) a.pre_costs[center] = 0.0f;
         }
         h = transform_normal_to_ref(cam, a.planes[center]);
         const float depth = h.w;
-        h.w = distance_to_origin(cam, px, py, depth, h);
+        h.w = distance_to_origin(cam, cx, cy, depth, h);
     } else if (a.prior) {
         if (a.masks[center] > 0 && a.costs[center] >= 0.1f) {
             const float pert = 0.02f;
@@ -599,7 +825,7 @@ __device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, WinWe
             const float lo = (1 - 3 * pert) * dp;
             const float hi = (1 + 3 * pert) * dp;
             dp = rng.uniform() * (hi - lo) + lo;
-            h = perturbed_normal(cam, px, py, hp, rng, (float)(3 * pert * kPiD));
+            h = perturbed_normal(cam, cx, cy, hp, rng, (float)(3 * pert * kPiD));
             h.w = dp;
         } else {
             /* the previous pass's world-frame normal, reused as it is
@@ -607,32 +833,35 @@ __device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, WinWe
              * reference frame first, as the geometric branch does */
             h = a.fix_quirks ? transform_normal_to_ref(cam, a.planes[center]) : a.planes[center];
             const float depth = h.w;
-            h.w = distance_to_origin(cam, px, py, depth, h);
+            h.w = distance_to_origin(cam, cx, cy, depth, h);
         }
     } else {
         const float depth = rng.uniform() * (a.dmax - a.dmin) + a.dmin;
-        h = random_normal(cam, px, py, rng, depth);
-        h.w = distance_to_origin(cam, px, py, depth, h);
+        h = random_normal(cam, cx, cy, rng, depth);
+        h.w = distance_to_origin(cam, cx, cy, depth, h);
     }
     float *cv = sCV + tid;
-    cost_vector(a, px, py, h, sWW, tid, rs, cv, kBlock);
+    cost_vector(a, px, py, act, h, win, rs, cv, kBlock);
+    if (!act) return;
     uint32_t sel;
     const float c = initial_cost_from(a, cv, kBlock, &sel);
     a.planes[center] = h;
     a.costs[center] = c;
     a.views[center] = sel;
     if (a.cost_cache) {
-        const Slot sl = slot_of(a, px, py);
+        const Slot sl = slot_of(a, cx, cy);
         for (int v = 0; v < a.n - 1; ++v) *cache_at(a, v, sl) = cv[v * kBlock];
     }
 }
 
 __global__ void __launch_bounds__(kBlock) k_init(const __grid_constant__ PMArgs a)
 {
-    __shared__ WinWeight sWW[kTaps * kBlock];
+    __shared__ float2 sW[kTaps / 2 * kBlock];
     __shared__ float sCV[kMaxSrc * kBlock];
+    __shared__ Spatial sp;
+    spatial_terms(a.sigma_spatial, &sp);
     const int tid = threadIdx.y * kBlockX + threadIdx.x;
-    init_body(a, blockIdx.x * kBlockX + threadIdx.x, blockIdx.y * kBlockY + threadIdx.y, sWW, sCV, tid);
+    init_body(a, blockIdx.x * kBlockX + threadIdx.x, blockIdx.y * kBlockY + threadIdx.y, sp, sW, sCV, tid);
 }
 
 /* Validity of the first site of direction k at extension round r (HPM.cu:1252-1445 and the
@@ -731,17 +960,20 @@ __device__ __forceinline__ bool same_plane(float4 p, float4 q)
            __float_as_uint(p.z) == __float_as_uint(q.z) && __float_as_uint(p.w) == __float_as_uint(q.w);
 }
 
-/* One red/black half-step runs as two kernels that hand the per-pixel cost
+/* One red/black half-step runs as three kernels that hand the per-pixel cost
  * matrix over through L2 instead of holding it in shared memory for the
  * whole pixel update (8 x S floats per pixel is what limits occupancy):
  *
  *   k_prop_dirs    NESP site choice, direction cost vectors, extension
  *                  (HPM.cu:1222-1543)
- *   k_prop_refine  joint view selection, candidate choice and
- *                  PlaneHypothesisRefinement (HPM.cu:1548-1725, 1143-1220)
+ *   k_prop_select  joint view selection and candidate choice
+ *                  (HPM.cu:1548-1725)
+ *   k_prop_refine  PlaneHypothesisRefinement (HPM.cu:1143-1220)
  *
- * The other colour is read-only during both kernels, so splitting the pixel
- * update changes nothing in what is computed. */
+ * The selection is one thread per pixel with an array per view in registers;
+ * between the window loops of the other two its code alone pushed them out of
+ * the instruction cache.  The other colour is read-only during all three, so
+ * splitting the pixel update changes nothing in what is computed. */
 
 #define CAG(k, v) a.cand_costs[(size_t)((k) * S + (v)) * sl.nh + sl.hc]
 /* Hand-off stores use the streaming cache policy (st.global.cs, evict
@@ -770,13 +1002,27 @@ __device__ __forceinline__ float dir_cost(const PMArgs &a, uint32_t code, int k,
     return (a.fix_quirks || (k == 0 && v == 0)) ? 2.0f : 0.0f; /* fix_quirks: the intended {2, 2, ...} */
 }
 
-__device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, int px, int py, WinPair *sWW, int tid)
+/* The windows that a warp still has to score, packed: lanes take them 32 at a
+ * time whatever pixel they belong to, so that a pixel with few distinct
+ * candidates leaves no idle lanes.  pos[k][lane]: the site of candidate k of
+ * the warp's pixel `lane`; item: candidate << 5 | lane. */
+struct DirItems {
+    int pos[8][32];
+    uint8_t item[8 * 32];
+};
+
+template <int WW>
+__device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const Patch<WW> &patch, DirItems &items)
 {
-    if (px >= a.W || py >= a.rows_cov) return;
     const int W = a.W, H = a.H, S = a.n - 1;
-    const int center = py * W + px;
-    const Slot sl = slot_of(a, px, py);
-    const RefStats rs = ref_window(a, px, py, sWW, tid);
+    const int lane = threadIdx.x, q0 = threadIdx.y * kBlockX;
+    const int px = patch.x(q0 + lane), py = patch.y(q0 + lane);
+    const bool act = px < W && py < a.rows_cov;
+    /* lanes outside the image stay for the warp's windows, on a pixel inside */
+    const int cx = min(px, W - 1), cy = min(py, H - 1);
+    const int center = cy * W + cx;
+    const Slot sl = slot_of(a, cx, cy);
+    const RefStats rs = ref_window(patch.win(q0 + lane));
     const float4 cur = a.planes[center];
 
     int pos[8];
@@ -797,9 +1043,10 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, int px
     uint32_t eval_mask = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        if (!first_site_valid(k, 0, px, py, W, H)) continue;
+        if (!act || !first_site_valid(k, 0, px, py, W, H)) continue;
         flags |= 1u << k;
         pos[k] = select_site(a, k, 0, px, py);
+        items.pos[k][lane] = pos[k];
         const float4 c = a.planes[pos[k]];
         uint32_t src = same_plane(c, cur) ? kRowCache : kRowNone;
 #pragma unroll
@@ -812,66 +1059,92 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, int px
         code = (code & ~(15u << (4 * k))) | (src << (4 * k));
     }
     /* 2) the distinct candidates, view by view, so that the threads of a
-     * block sample one source image at a time (texture-cache locality) */
-    for (int v = 0; v < S; ++v) {
-        uint32_t m = eval_mask;
-        while (m) {
-            const int k = __ffs(m) - 1;
-            m &= m - 1;
-            CAG_PUT(k, v, ncc_call(a, v + 1, px, py, a.planes[pos[k]], sWW, tid, rs));
-        }
-    }
-    if (a.counters && eval_mask) atomicAdd(&a.counters[0], (unsigned long long)(__popc(eval_mask) * S));
-
-    /* Extension: only the left-up polyline can extend, because
+     * block sample one source image at a time (texture-cache locality).
+     * Round 0 scores the sites; rounds 1 to 3 are the extension.
+     * Extension: only the left-up polyline can extend, because
      * bool symbol_eight_orientations[10] = { true } sets index 0 only
      * (HPM.cu:1475).  JudgeExtend: HPM.cu:1036-1059. */
-    if (flags & 1u) {
-        bool detached = false; /* rows that copy direction 0's first row hold their own copy */
-        for (int r = 0; r < 3; ++r) {
+    bool extend = (flags & 1u) != 0;
+    bool detached = false; /* rows that copy direction 0's first row hold their own copy */
+#pragma unroll 1
+    for (int round = 0; round < 4; ++round) {
+        if (round > 0) {
+            const int r = round - 1;
+            eval_mask = 0;
+            if (!__any_sync(kAll, extend)) break;
+            __syncwarp(); /* the rows scored by other lanes */
             const float good = (float)(0.8 * exp(-iter * iter * (3 - r) / 90.0));
-            int good_sum = 0, bad_sum = 0;
-            for (int v = 0; v < S; ++v) {
-                const float c = dir_cost(a, code, 0, v, S, sl);
-                if (c < good) good_sum++;
-                if (c > 1.2f) bad_sum++;
+            if (extend) {
+                int good_sum = 0, bad_sum = 0;
+                for (int v = 0; v < S; ++v) {
+                    const float c = dir_cost(a, code, 0, v, S, sl);
+                    if (c < good) good_sum++;
+                    if (c > 1.2f) bad_sum++;
+                }
+                if (good_sum >= 1 && bad_sum <= 2) extend = false;
             }
-            if (good_sum >= 1 && bad_sum <= 2) break;
-            if (!first_site_valid(0, r, px, py, W, H)) continue; /* flag[0] is set: keep site and costs */
-            const int best = select_site(a, 0, r, px, py);
-            if (a.costs[best] > a.costs[pos[0]]) continue; /* the previous site is better: keep it */
-            const float4 prev = a.planes[pos[0]];
-            pos[0] = best;
-            const float4 p = a.planes[best];
-            if (same_plane(p, prev)) continue;
-            /* direction 0's row changes: the rows that refer to it keep the
-             * values it had when they were chosen */
-            if (!detached) {
-                detached = true;
+            /* an invalid first site keeps site and costs: flag[0] is set */
+            if (extend && first_site_valid(0, r, px, py, W, H)) {
+                const int best = select_site(a, 0, r, px, py);
+                /* a better previous site is kept */
+                if (!(a.costs[best] > a.costs[pos[0]])) {
+                    const float4 prev = a.planes[pos[0]];
+                    pos[0] = best;
+                    items.pos[0][lane] = best;
+                    const float4 p = a.planes[best];
+                    if (!same_plane(p, prev)) {
+                        /* direction 0's row changes: the rows that refer to
+                         * it keep the values it had when they were chosen */
+                        if (!detached) {
+                            detached = true;
 #pragma unroll
-                for (int k = 1; k < 8; ++k)
-                    if (((code >> (4 * k)) & 15u) == 0u) {
-                        for (int v = 0; v < S; ++v) CAG_PUT(k, v, dir_cost(a, code, 0, v, S, sl));
-                        code = (code & ~(15u << (4 * k))) | (kRowOwn << (4 * k));
+                            for (int k = 1; k < 8; ++k)
+                                if (((code >> (4 * k)) & 15u) == 0u) {
+                                    for (int v = 0; v < S; ++v) CAG_PUT(k, v, dir_cost(a, code, 0, v, S, sl));
+                                    code = (code & ~(15u << (4 * k))) | (kRowOwn << (4 * k));
+                                }
+                        }
+                        int src = -1;
+#pragma unroll
+                        for (int j = 1; j < 8; ++j)
+                            if (src < 0 && ((flags >> j) & 1u) && same_plane(p, a.planes[pos[j]])) src = j;
+                        if (same_plane(p, cur)) {
+                            code = (code & ~15u) | kRowCache;
+                        } else if (src >= 0) {
+                            const uint32_t sj = (code >> (4 * src)) & 15u;
+                            code = (code & ~15u) | (sj == kRowOwn ? (uint32_t)src : sj);
+                        } else {
+                            eval_mask = 1u;
+                            code = (code & ~15u) | kRowOwn;
+                        }
                     }
-            }
-            if (same_plane(p, cur)) {
-                code = (code & ~15u) | kRowCache;
-                continue;
-            }
-            int src = -1;
-#pragma unroll
-            for (int j = 1; j < 8; ++j)
-                if (src < 0 && ((flags >> j) & 1u) && same_plane(p, a.planes[pos[j]])) src = j;
-            if (src >= 0) {
-                const uint32_t sj = (code >> (4 * src)) & 15u;
-                code = (code & ~15u) | (sj == kRowOwn ? (uint32_t)src : sj);
-            } else {
-                cost_vector(a, px, py, p, sWW, tid, rs, &CAG(0, 0), (int)sl.nh);
-                code = (code & ~15u) | kRowOwn;
+                }
             }
         }
+        int total = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const unsigned m = __ballot_sync(kAll, (eval_mask >> k) & 1u);
+            if ((eval_mask >> k) & 1u) items.item[total + __popc(m & lanes_below())] = (uint8_t)(k << 5 | lane);
+            total += __popc(m);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int v = 0; v < S; ++v)
+#pragma unroll 1
+            for (int base = 0; base < total; base += 32) {
+                const bool need = base + lane < total;
+                const int it = items.item[need ? base + lane : 0], k = it >> 5, p = it & 31, q = q0 + p;
+                const RefStats st = stats_of(rs, p);
+                const int hc = __shfl_sync(kAll, sl.hc, p);
+                const float c = ncc_quad(a, v + 1, patch.x(q), patch.y(q), need, a.planes[items.pos[k][p]],
+                                         patch.win(q), st);
+                if (need) __stcs(&a.cand_costs[(size_t)(k * S + v) * sl.nh + hc], c);
+            }
+        if (a.counters && eval_mask) atomicAdd(&a.counters[0], (unsigned long long)(__popc(eval_mask) * S));
     }
+    __syncwarp();
+    if (!act) return;
     /* 3) every valid direction's row in its own slot: a row that refers to
      * the cost-vector cache or to an earlier direction (always one that owns
      * its row) is copied there, so that the refinement reads each row with
@@ -894,25 +1167,30 @@ template <int WW>
 __global__ void __launch_bounds__(kBlock, HPM_P1_MIN_BLOCKS) k_prop_dirs(const __grid_constant__ PMArgs a, int iter,
                                                                           int color)
 {
-    __shared__ WinPair sWW[kTaps * kBlock];
-    const int tid = threadIdx.y * kBlockX + threadIdx.x;
-    int px, py;
-    half_step_pixel_at(blockIdx.x, blockIdx.y, WW, color, px, py);
-    prop_dirs_body(a, iter, px, py, sWW, tid);
+    __shared__ PatchMem<WW> sPatch;
+    __shared__ DirItems sItems[kBlockY];
+    prop_dirs_body(a, iter, sPatch.load(a, color), sItems[threadIdx.y]);
 }
 
-/* PROP: the prior-net form, whose network proposal a.proposals[center] is a
- * sixth refinement candidate, scored by the same NCC (and prior terms) as the
- * other five and accepted by the same rule.  It takes no random draws, so
- * the random stream of the other candidates is unchanged.
- * ACMM: the ACMM+NESP variant (ACMM.cu:1548-1629, 623-667): geometric weight
- * 0.2 on the current and refined hypotheses, no NaN fallback, and in a
- * hierarchy pass the threshold rule on the result.  A separate
- * instantiation, so that the HPM-MVS kernels keep their registers. */
-template <int SMAX, bool PROP, bool ACMM>
-__device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int px, int py, WinPair *sWW, int tid)
+/* What the selection hands to the refinement, per pixel (rf_* in PMArgs):
+ * plane and (cost, its depth, its restricted cost, the current hypothesis's
+ * cost) after the neighbours, the view weights (at most 15 draws, 4 bits per
+ * view) and the row of the cost vector that belongs to the plane.
+ * ACMM: the ACMM+NESP variant (ACMM.cu:1548-1629): geometric weight 0.2 on
+ * the current hypothesis, no NaN fallback.  A separate instantiation. */
+constexpr int kRowCurrent = 15;
+constexpr int kViewDraws = 15; /* HPM.cu:1590 */
+
+/* weight of view v: 4 bits each, 16 views per word */
+__device__ __forceinline__ float view_weight(unsigned long long lo, unsigned long long hi, int v)
 {
-    constexpr float kGeomW = ACMM ? 0.2f : 0.1f; /* HPM.cu:1642, 1189; ACMM.cu:1596, 651 */
+    return (float)((v < 16 ? lo >> (4 * v) : hi >> (4 * (v - 16))) & 15ull);
+}
+
+template <int SMAX, bool ACMM>
+__device__ __forceinline__ void prop_select_body(const PMArgs &a, int iter, int px, int py)
+{
+    constexpr float kGeomW = ACMM ? 0.2f : 0.1f; /* HPM.cu:1642; ACMM.cu:1596 */
     if (px >= a.W || py >= a.rows_cov) return;
     const int W = a.W, S = a.n - 1;
     const int center = py * W + px;
@@ -982,7 +1260,7 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
                 sp[v] = cum;
             }
     }
-    for (int smp = 0; smp < 15; ++smp) {
+    for (int smp = 0; smp < kViewDraws; ++smp) {
         const float rp = rng.uniform() - FLT_EPSILON;
         bool done = false;
 #pragma unroll
@@ -993,7 +1271,6 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
             }
         }
     }
-    uint32_t tsv = 0;
     float wn = 0.0f;
     /* the integer view weights, 4 bits per view (at most 15 draws), for
      * loops over the selected views with a run-time index */
@@ -1001,7 +1278,6 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
 #pragma unroll
     for (int v = 0; v < SMAX; ++v)
         if (v < S && vw[v] > 0) {
-            tsv |= 1u << v;
             wn += vw[v];
             if (v < 16)
                 vw_lo |= (unsigned long long)vw[v] << (4 * v);
@@ -1057,7 +1333,7 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
     }
     cost_now /= wn;
     float cost = cost_now;
-    uint32_t sel = a.views[center];
+    bool sel_new = false; /* the selected views change to the weighted ones */
     float depth_now = depth_from_plane(cam, plane, px, py);
 
     float restricted_cost = 0.0f;
@@ -1103,7 +1379,7 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
                     best_row = max_idx;
                     cost = fc[max_idx];
                     restricted_cost = rfc[max_idx];
-                    sel = tsv;
+                    sel_new = true;
                 }
             }
         } else if (FLAG(min_idx)) {
@@ -1125,18 +1401,97 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
             plane = hb;
             best_row = min_idx;
             cost = fc[min_idx];
-            sel = tsv;
+            sel_new = true;
         }
         if (!ACMM && cost != cost) { /* the ACMM+NESP variant has no such fallback */
             depth_now = db;
             plane = hb;
             best_row = min_idx;
-            sel = tsv;
+            sel_new = true;
         }
     }
 
+    a.rf_plane[sl.hc] = plane;
+    a.rf_state[sl.hc] = make_float4(cost, depth_now, restricted_cost, cost_now);
+    uint32_t *weights = a.rf_views + (size_t)sl.hc * (SMAX > 16 ? 4 : 2);
+    weights[0] = (uint32_t)vw_lo;
+    weights[1] = (uint32_t)(vw_lo >> 32);
+    if constexpr (SMAX > 16) {
+        weights[2] = (uint32_t)vw_hi;
+        weights[3] = (uint32_t)(vw_hi >> 32);
+    }
+    /* the direction's flags are read for the last time above */
+    a.cand_flags[sl.hc] = (uint32_t)(best_row < 0 ? kRowCurrent : best_row) | (sel_new ? 16u : 0u);
+#undef ROWC
+#undef FLAG
+}
+
+template <int SMAX, int WW, bool ACMM>
+__global__ void __launch_bounds__(kBlock) k_prop_select(const __grid_constant__ PMArgs a, int iter, int color)
+{
+    int px, py;
+    half_step_pixel_at(blockIdx.x, blockIdx.y, WW, color, px, py);
+    prop_select_body<SMAX, ACMM>(a, iter, px, py);
+}
+
+/* Shared memory of the refinement, per warp: its pixels' candidate planes and
+ * the weighted sums of their costs; per block, the pixels whose winner's cost vector is
+ * not complete yet. */
+template <int NC>
+struct RefineItems {
+    float4 cand[kBlockY][NC][32];
+    float cost[kBlockY][NC][32];
+    uint8_t rank[kBlockY][kBlock];
+    uint32_t missing[kBlock];
+};
+
+/* PROP: the prior-net form, whose network proposal a.proposals[center] is a
+ * sixth refinement candidate, scored by the same NCC (and prior terms) as the
+ * other five and accepted by the same rule.  It takes no random draws, so
+ * the random stream of the other candidates is unchanged.
+ * ACMM: the ACMM+NESP variant (ACMM.cu:623-667): geometric weight 0.2 on the
+ * refined hypotheses, and in a hierarchy pass the threshold rule on the
+ * result.  A separate instantiation. */
+template <bool PROP, bool ACMM, int WW>
+__device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, const Patch<WW> &patch,
+                                                 RefineItems<PROP ? 6 : 5> &items)
+{
+    constexpr float kGeomW = ACMM ? 0.2f : 0.1f; /* HPM.cu:1189; ACMM.cu:651 */
+    constexpr int NC = PROP ? 6 : 5;
+    const int W = a.W, S = a.n - 1;
+    const int lane = threadIdx.x, wv = threadIdx.y, q0 = wv * kBlockX;
+    int px = patch.x(q0 + lane), py = patch.y(q0 + lane);
+    const bool act = px < W && py < a.rows_cov;
+    /* lanes outside the image stay for the block's windows, on a pixel
+     * inside, with no view weight and no write */
+    px = min(px, W - 1);
+    py = min(py, a.H - 1);
+    const int center = py * W + px;
+    const Slot sl = slot_of(a, px, py);
+    const HpmCamera &cam = a.cam[0];
     /* PlaneHypothesisRefinement, HPM.cu:1143-1220 */
-    const RefStats rs = ref_window(a, px, py, sWW, tid);
+    const RefStats rs = ref_window(patch.win(q0 + lane));
+    float4 plane = a.rf_plane[sl.hc];
+    const float4 state = a.rf_state[sl.hc];
+    float cost = state.x, depth_now = state.y, restricted_cost = state.z;
+    const uint32_t row_code = a.cand_flags[sl.hc];
+    int best_row = (int)(row_code & 15u); /* kRowCurrent: the cached current hypothesis */
+    unsigned long long vw_lo = 0, vw_hi = 0;
+    if (act) {
+        const uint32_t *weights = a.rf_views + (size_t)sl.hc * (S > 16 ? 4 : 2);
+        vw_lo = weights[0] | (unsigned long long)weights[1] << 32;
+        if (S > 16) vw_hi = weights[2] | (unsigned long long)weights[3] << 32;
+    }
+    /* the selected views and the sum of their (integer) weights */
+    uint32_t tsv = 0;
+    float wn = 0.0f;
+    for (int v = 0; v < S; ++v) {
+        const float w = view_weight(vw_lo, vw_hi, v);
+        if (w > 0) tsv |= 1u << v;
+        wn += w;
+    }
+    Rng rng;
+    rng.resume(a.seed_lo, a.seed_hi, (uint32_t)center, (uint32_t)(1 + iter), a.salt, kViewDraws);
     {
         const float pert = 0.02f;
         const float depth_sigma = (a.dmax - a.dmin) / 64.0f;
@@ -1172,51 +1527,64 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
          * across the warp (one source texture per texture instruction, one
          * source image at a time per block); each NCC value goes to the
          * candidate's hand-off row for the cache. */
-        constexpr int NC = PROP ? 6 : 5;
-        float4 cand[NC];
         float cand_depth[NC];
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
-            cand[i] = normals[i];
-            cand[i].w = distance_to_origin(cam, px, py, depths[i], cand[i]);
+            float4 c = normals[i];
+            c.w = distance_to_origin(cam, px, py, depths[i], c);
+            items.cand[wv][i][lane] = c;
             cand_depth[i] = depths[i];
         }
         if constexpr (PROP) {
-            cand[5] = a.proposals[center];
-            cand_depth[5] = depth_from_plane(cam, cand[5], px, py);
+            const float4 c = a.proposals[center];
+            items.cand[wv][5][lane] = c;
+            cand_depth[5] = depth_from_plane(cam, c, px, py);
         }
-        float tc[NC];
 #pragma unroll
-        for (int i = 0; i < NC; ++i) tc[i] = 0.0f;
-        for (int v = 0; v < S; ++v) {
-            const bool selected = (tsv >> v) & 1u;
-            const float w = (float)((v < 16 ? (vw_lo >> (4 * v)) : (vw_hi >> (4 * (v - 16)))) & 15ull);
+        for (int i = 0; i < NC; ++i) items.cost[wv][i][lane] = 0.0f;
 #pragma unroll 1
-            for (int k = 0; k < NC; ++k) {
-                /* candidates 0 and 2 share the random depth, hence the window
-                 * centre in every source view; 1, 3 and 4 sit at or near the
-                 * current depth: scoring 0, 2, 1, 3, 4 keeps windows with the
-                 * same centre back to back in the texture cache */
-                const int i = (0x543120 >> (4 * k)) & 15;
-                const float c = ncc_call(a, v + 1, px, py, cand[i], sWW, tid, rs);
-                CAG_PUT(kRefineRow + i, v, c);
-                if (selected) {
-                    if (a.geom)
-                        tc[i] += w * (c + kGeomW * geom_cost(a, v + 1, cand[i], px, py));
-                    else
-                        tc[i] += w * c;
+        for (int v = 0; v < S; ++v) {
+            /* the candidates of the pixels that weigh this view, packed: a
+             * pixel's together, candidates 0 and 2 (which share the random
+             * depth, hence the window centre) and 1, 3, 4 (at or near the
+             * current depth) next to each other, so that windows with the
+             * same centre meet in the texture cache */
+            const float weight = view_weight(vw_lo, vw_hi, v);
+            const bool selected = weight > 0.0f;
+            const unsigned m = __ballot_sync(kAll, selected);
+            if (m == 0) continue;
+            const int total = __popc(m) * NC;
+            if (selected) items.rank[wv][__popc(m & lanes_below())] = (uint8_t)lane;
+            __syncwarp();
+#pragma unroll 1
+            for (int base = 0; base < total; base += 32) {
+                const bool need = base + lane < total;
+                const int j = need ? base + lane : 0, n = j / NC, p = items.rank[wv][n], q = q0 + p;
+                const int i = (0x543120 >> (4 * (j - n * NC))) & 15;
+                const RefStats st = stats_of(rs, p);
+                const int hc = __shfl_sync(kAll, sl.hc, p);
+                const float w = __shfl_sync(kAll, weight, p);
+                const float4 h = items.cand[wv][i][p];
+                const int qx = patch.x(q), qy = patch.y(q);
+                float c = ncc_quad(a, v + 1, qx, qy, need, h, patch.win(q), st);
+                if (need) {
+                    __stcs(&a.cand_costs[(size_t)((kRefineRow + i) * S + v) * sl.nh + hc], c);
+                    if (a.geom) c = __fmaf_rn(kGeomW, geom_cost(a, v + 1, h, qx, qy), c);
+                    items.cost[wv][i][p] = __fmaf_rn(w, c, items.cost[wv][i][p]);
                 }
             }
+            __syncwarp();
         }
-        if (a.counters) atomicAdd(&a.counters[0], (unsigned long long)(NC * S));
+        if (a.counters && tsv) atomicAdd(&a.counters[0], (unsigned long long)(NC * __popc(tsv)));
 #pragma unroll
         for (int i = 0; i < NC; ++i) {
-            const float tci = tc[i] / wn;
-            const float depth_before = depth_from_plane(cam, cand[i], px, py);
+            const float tci = items.cost[wv][i][lane] / wn;
+            const float4 ci = items.cand[wv][i][lane];
+            const float depth_before = depth_from_plane(cam, ci, px, py);
             bool take;
             if (use_prior) {
                 const float dd = cand_depth[i] - depth_prior;
-                const float pr = restricted_prior(dd, dot3(pp, cand[i]), two_dss, two_ass);
+                const float pr = restricted_prior(dd, dot3(pp, ci), two_dss, two_ass);
                 const float rtc = expf(-tci * tci / beta) * pr;
                 take = depth_before >= a.dmin && depth_before <= a.dmax && rtc > restricted_cost;
                 if (take) restricted_cost = rtc;
@@ -1225,7 +1593,7 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
             }
             if (take) {
                 depth_now = depth_before;
-                plane = cand[i];
+                plane = ci;
                 cost = tci;
                 best_row = kRefineRow + i;
             }
@@ -1237,32 +1605,62 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, int 
      * weights (its selected views may still have changed) */
     if constexpr (ACMM) {
         if (a.pre_costs && !(cost < a.pre_costs[center] - 0.1f)) {
-            plane = cur;
-            cost = cost_now;
-            best_row = -1;
+            plane = a.planes[center];
+            cost = state.w;
+            best_row = kRowCurrent;
         }
     }
+    /* the winner's cost vector for the cache: the views without a weight have
+     * not been scored for the refinement candidates.  They are few, so both
+     * warps' are packed together, and the views dealt out to the warps. */
+    const bool took = act && best_row >= kRefineRow && best_row != kRowCurrent;
+    const uint32_t all = S == 32 ? kAll : (1u << S) - 1u;
+    __syncthreads();
+    items.cand[wv][0][lane] = plane;
+    items.cost[wv][0][lane] = rs.inv;
+    items.cost[wv][1][lane] = rs.mean;
+    items.cost[wv][2][lane] = rs.var;
+    items.missing[q0 + lane] = took ? all & ~tsv : 0u;
+    __syncthreads();
+#pragma unroll 1
+    for (int v = wv; v < S; v += kBlockY) {
+        int total = 0;
+#pragma unroll
+        for (int half = 0; half < kBlockY; ++half) {
+            const bool mine = (items.missing[half * kBlockX + lane] >> v) & 1u;
+            const unsigned m = __ballot_sync(kAll, mine);
+            if (mine) items.rank[wv][total + __popc(m & lanes_below())] = (uint8_t)(half * kBlockX + lane);
+            total += __popc(m);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int base = 0; base < total; base += 32) {
+            const bool need = base + lane < total;
+            const int q = need ? items.rank[wv][base + lane] : 0, qw = q >> 5, p = q & 31;
+            const RefStats st = {items.cost[qw][0][p], items.cost[qw][1][p], items.cost[qw][2][p]};
+            const int qx = patch.x(q), qy = patch.y(q);
+            const float c = ncc_quad(a, v + 1, qx, qy, need, items.cand[qw][0][p], patch.win(q), st);
+            if (need) *cache_at(a, v, slot_of(a, qx, qy)) = c;
+        }
+        __syncwarp();
+    }
+    if (a.counters && took) atomicAdd(&a.counters[0], (unsigned long long)(S - __popc(tsv)));
+    if (!act) return;
     a.planes[center] = plane;
     a.costs[center] = cost;
-    a.views[center] = sel;
-    if (best_row >= kRefineRow) {
-        for (int v = 0; v < S; ++v) *cache_at(a, v, sl) = CAG(best_row, v);
-    } else if (best_row >= 0) {
-        for (int v = 0; v < S; ++v) *cache_at(a, v, sl) = CAG(best_row, v);
-    }
-#undef ROWC
-#undef FLAG
+    if (row_code & 16u) a.views[center] = tsv;
+    if (best_row == kRowCurrent) return;
+    for (int v = 0; v < S; ++v)
+        if (!took || ((tsv >> v) & 1u)) *cache_at(a, v, sl) = CAG(best_row, v);
 }
 
-template <int SMAX, bool PROP, int WW, bool ACMM = false>
+template <bool PROP, int WW, bool ACMM>
 __global__ void __launch_bounds__(kBlock, HPM_P2_MIN_BLOCKS) k_prop_refine(const __grid_constant__ PMArgs a, int iter,
                                                                             int color)
 {
-    __shared__ WinPair sWW[kTaps * kBlock];
-    const int tid = threadIdx.y * kBlockX + threadIdx.x;
-    int px, py;
-    half_step_pixel_at(blockIdx.x, blockIdx.y, WW, color, px, py);
-    prop_refine_body<SMAX, PROP, ACMM>(a, iter, px, py, sWW, tid);
+    __shared__ PatchMem<WW> sPatch;
+    __shared__ RefineItems<PROP ? 6 : 5> sItems;
+    prop_refine_body<PROP, ACMM, WW>(a, iter, sPatch.load(a, color), sItems);
 }
 #undef CAG_PUT
 #undef CAG
@@ -1321,30 +1719,38 @@ __global__ void k_filter(const __grid_constant__ PMArgs a, float4 *pl, const flo
 __global__ void __launch_bounds__(kBlock) k_cost_vectors(const __grid_constant__ PMArgs a, const float4 *planes,
                                                           float *out)
 {
-    __shared__ WinPair sWW[kTaps * kBlock];
+    __shared__ float2 sW[kTaps / 2 * kBlock];
+    __shared__ Spatial sp;
+    spatial_terms(a.sigma_spatial, &sp);
     const int tid = threadIdx.y * kBlockX + threadIdx.x;
     const int px = blockIdx.x * kBlockX + threadIdx.x;
     const int py = blockIdx.y * kBlockY + threadIdx.y;
-    if (px >= a.W || py >= a.H) return;
-    const RefStats rs = ref_window(a, px, py, sWW, tid);
-    const int c = py * a.W + px;
+    const bool act = px < a.W && py < a.H;
+    const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
+    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
+    const RefStats rs = ref_window(win);
+    const int c = cy * a.W + cx;
     const int S = a.n - 1;
-    cost_vector(a, px, py, planes[c], sWW, tid, rs, out + (size_t)c * S, 1);
+    cost_vector(a, px, py, act, planes[c], win, rs, out + (size_t)c * S, 1);
 }
 
 __global__ void __launch_bounds__(kBlock) k_initial_costs(const __grid_constant__ PMArgs a, const float4 *planes,
                                                           float *cost, uint32_t *views)
 {
-    __shared__ WinPair sWW[kTaps * kBlock];
+    __shared__ float2 sW[kTaps / 2 * kBlock];
+    __shared__ Spatial sp;
+    spatial_terms(a.sigma_spatial, &sp);
     __shared__ float sCV[kMaxSrc * kBlock];
     const int tid = threadIdx.y * kBlockX + threadIdx.x;
     const int px = blockIdx.x * kBlockX + threadIdx.x;
     const int py = blockIdx.y * kBlockY + threadIdx.y;
-    if (px >= a.W || py >= a.H) return;
-    const RefStats rs = ref_window(a, px, py, sWW, tid);
-    const int c = py * a.W + px;
-    cost_vector(a, px, py, planes[c], sWW, tid, rs, sCV + tid, kBlock);
-    cost[c] = initial_cost_from(a, sCV + tid, kBlock, &views[c]);
+    const bool act = px < a.W && py < a.H;
+    const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
+    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
+    const RefStats rs = ref_window(win);
+    const int c = cy * a.W + cx;
+    cost_vector(a, px, py, act, planes[c], win, rs, sCV + tid, kBlock);
+    if (act) cost[c] = initial_cost_from(a, sCV + tid, kBlock, &views[c]);
 }
 
 __global__ void k_geom_costs(const __grid_constant__ PMArgs a, const float4 *planes, float *out)
@@ -1373,11 +1779,14 @@ __global__ void k_tap_samples(const __grid_constant__ PMArgs a, const float4 *pl
     const float fpx = (float)px, fpy = (float)py;
     const float2 pt = warp(H, fpx, fpy);
     inside[k] = !(pt.x >= sc.width || pt.x < 0.0f || pt.y >= sc.height || pt.y < 0.0f);
-    int t = 0;
 #pragma unroll
-    for (int i = -5; i < 6; i += 2)
+    for (int tp = 0; tp < 4; ++tp) {
+        float s[9];
+        fetch_block(a.view[v].tex, H, fpx + (float)(2 * (tp & 1) - 5), fpy + (float)(2 * (tp >> 1) - 5), s);
 #pragma unroll
-        for (int j = -5; j < 6; j += 2, ++t) out[(size_t)k * kTaps + t] = tap_sample(a.view[v].tex, H, fpx, fpy, i, j);
+        for (int b = 0; b < 9; ++b)
+            out[(size_t)k * kTaps + (2 * (b / 3) + (tp & 1)) * 6 + 2 * (b % 3) + (tp >> 1)] = s[b];
+    }
 }
 
 template <int SMAX, int WW>
@@ -1388,14 +1797,16 @@ cudaError_t launch_prop_t(const PMArgs &a, int iter, int color, cudaStream_t s)
     k_prop_dirs<WW><<<grid, b, 0, s>>>(a, iter, color);
     if constexpr (WW == 8) { /* the ACMM+NESP variant runs the default tile */
         if (a.acmm) {
-            k_prop_refine<SMAX, false, WW, true><<<grid, b, 0, s>>>(a, iter, color);
+            k_prop_select<SMAX, WW, true><<<grid, b, 0, s>>>(a, iter, color);
+            k_prop_refine<false, WW, true><<<grid, b, 0, s>>>(a, iter, color);
             return cudaGetLastError();
         }
     }
+    k_prop_select<SMAX, WW, false><<<grid, b, 0, s>>>(a, iter, color);
     if (a.proposals)
-        k_prop_refine<SMAX, true, WW><<<grid, b, 0, s>>>(a, iter, color);
+        k_prop_refine<true, WW, false><<<grid, b, 0, s>>>(a, iter, color);
     else
-        k_prop_refine<SMAX, false, WW><<<grid, b, 0, s>>>(a, iter, color);
+        k_prop_refine<false, WW, false><<<grid, b, 0, s>>>(a, iter, color);
     return cudaGetLastError();
 }
 

@@ -521,9 +521,10 @@ int hpm_profile_enable(hpm_ctx *ctx, int enable);
  * jbu]; counts = launches of each.  Either pointer may be NULL. */
 int hpm_profile_read(hpm_ctx *ctx, float *ms4, int *counts4);
 /* Work counters: bilateral NCC window evaluations (one per hypothesis and
- * source view) and geometric-consistency terms, summed over every pass run
- * since hpm_count_enable(ctx, 1), which zeroes them.  Diagnostic; no
- * reference counterpart. */
+ * source view that is scored; a refinement candidate is scored in the views
+ * its pixel weighs, the winner in the others too) and geometric-consistency
+ * terms, summed over every pass run since hpm_count_enable(ctx, 1), which
+ * zeroes them.  Diagnostic; no reference counterpart. */
 int hpm_count_enable(hpm_ctx *ctx, int enable);
 int hpm_count_read(hpm_ctx *ctx, uint64_t *ncc_windows, uint64_t *geom_terms);
 
