@@ -46,20 +46,20 @@ constexpr int kHaloBytes = 3 * kHaloW * 16; /* one channel group: 6240 B */
 constexpr int kSlab = 6272;                 /* slab stride, a multiple of 128 B */
 constexpr long long kWaitCycles = 4000000000LL; /* ~2 s at 2 GHz */
 
-/* Shared memory of one CTA.  The A region is large enough that every
- * address an MMA may read stays inside it even under the other reading of
- * the two stride fields (the M stride taken as the slab): a mistaken
- * descriptor gives wrong numbers, never an out-of-bounds access. */
+/* Shared memory of one CTA: the halo and the weights, nothing more, so that
+ * several CTAs share an SM and one's loads run under another's (a CTA is a
+ * chain: TMA, MMAs, epilogue).  The last tap's last core matrix ends inside
+ * its slab: (2 kHaloW + 2) * 16 + 15 * 128 + 128 <= kSlab.  At 400x300, 32 to
+ * 32 channels: 30 us with one CTA per SM (a halo region with slack), 15 us
+ * with five. */
 template <int CIN, int COUT>
 struct ConvSmem {
     static constexpr int CG = CIN / 8, OG = COUT / 8;
-    static constexpr int kAStartMax = (CG - 2 > 0 ? CG - 2 : 0) * kSlab + (2 * kHaloW + 2) * 16;
-    static constexpr int kAReach = kAStartMax + 15 * kSlab + 2 * 128 + 128;
-    static constexpr int kA = ((kAReach > CG * kSlab ? kAReach : CG * kSlab) + 1023) / 1024 * 1024;
+    static constexpr int kA = (CG * kSlab + 1023) / 1024 * 1024;
     static constexpr int kB = 9 * CIN * COUT * 2;
-    static constexpr int kBReach = ((8 * CG + CG - 2 > 0 ? 8 * CG + CG - 2 : 0) * OG) * 128 + OG * OG * 128 + 256;
-    static constexpr int kBRegion = ((kBReach > kB ? kBReach : kB) + 1023) / 1024 * 1024;
+    static constexpr int kBRegion = (kB + 1023) / 1024 * 1024;
     static constexpr int kBytes = kA + kBRegion + 64;
+    static_assert((2 * kHaloW + 2) * 16 + 15 * 128 + 128 <= kSlab, "the last tap ends inside its slab");
 };
 
 enum { kEpiReluBf16 = 0, kEpiBiasF32 = 1, kEpiDreluBf16 = 2 };
@@ -74,7 +74,7 @@ __device__ __forceinline__ void load_acc(uint32_t taddr, uint32_t *r)
 }
 
 template <int CIN, int COUT, int EPI, bool TMA>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(128)
     k_conv3x3(const __grid_constant__ CUtensorMap tmap, const __nv_bfloat16 *__restrict__ x, int h, int w,
               const uint4 *__restrict__ wpk, const float *__restrict__ bias, const __nv_bfloat16 *__restrict__ aux,
               void *__restrict__ y, int *__restrict__ err)
@@ -167,7 +167,10 @@ __global__ void __launch_bounds__(128, 1)
                         v[n / 2] = __floats2bfloat162_rn(fmaxf(__uint_as_float(r[n]) + bias[n], 0.0f),
                                                          fmaxf(__uint_as_float(r[n + 1]) + bias[n + 1], 0.0f));
                 } else {
-                    const __nv_bfloat16 *ax = aux + o;
+                    __align__(16) __nv_bfloat16 ax[COUT];
+#pragma unroll
+                    for (int q = 0; q < COUT / 8; ++q)
+                        reinterpret_cast<uint4 *>(ax)[q] = reinterpret_cast<const uint4 *>(aux + o)[q];
 #pragma unroll
                     for (int n = 0; n < COUT; n += 2) {
                         const float g0 = __bfloat162float(ax[n]) > 0.0f ? __uint_as_float(r[n]) : 0.0f;
@@ -203,29 +206,36 @@ __global__ void __launch_bounds__(128, 1)
  *       kgroup * OG * 128.
  * A persistent CTA walks its 128-pixel row tiles and accumulates NG
  * accumulators of 128 x COUT in TMEM across all of them, then adds them to
- * dW (FP32, OIHW) with atomics. */
+ * dW (FP32, OIHW) with atomics.  What bounds it is staging A (96 KB a tile)
+ * and the atomics: 512 threads load A, all of a thread's loads in flight
+ * together, and two CTAs share an SM, so that one stages while the other's
+ * MMAs run (400x300, 32 to 32 channels: 90 us with one CTA of 128 threads, 28
+ * us now; one CTA of 512 per SM 35 us).  The bias gradient is summed from the
+ * dY tile on its way to shared memory: a thread always loads the same 8
+ * channels (a kernel of its own took 92 us, nearly all of it atomics of every
+ * warp on 32 addresses). */
+constexpr int kWgradThreads = 512;
 template <int CIN, int COUT>
 struct WgradSmem {
     static constexpr int CG = CIN / 8, OG = COUT / 8, TG = 128 / CIN, NG = (9 + TG - 1) / TG;
     static constexpr int kAGroup = 16 * 16 * 128; /* 16 pixel groups x 16 m groups */
     static constexpr int kA = NG * kAGroup;
-    static constexpr int kB = 16 * OG * 128 + 1024; /* + reach of the other stride reading */
-    /* under the other reading of the two strides the last A group reaches
-     * 7 * 4096 + 15 * 2048 + 255 bytes past its start: one group of slack */
-    static constexpr int kBytes = kA + kB + kAGroup + 64;
+    static constexpr int kB = 16 * OG * 128;
+    static constexpr int kBytes = kA + kB + COUT * 4 + 64;
 };
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(kWgradThreads, 2)
     k_conv_wgrad(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ dy, int h, int w,
-                 float *__restrict__ dw, int *__restrict__ err)
+                 float *__restrict__ dw, float *__restrict__ db, int *__restrict__ err)
 {
     using L = WgradSmem<CIN, COUT>;
     constexpr int CG = L::CG, OG = L::OG, TG = L::TG, NG = L::NG;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sA = smem;
     uint8_t *sB = smem + L::kA;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sB + L::kB + L::kAGroup);
+    float *sDb = reinterpret_cast<float *>(sB + L::kB);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sDb + COUT);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     static_assert(L::kBytes <= 227 * 1024, "shared memory of one CTA");
@@ -238,35 +248,52 @@ __global__ void __launch_bounds__(128, 1)
         tc::mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (tid < COUT) sDb[tid] = 0.0f;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    float bsum[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     const int tiles_x = (w + kTileM - 1) / kTileM, tiles = h * tiles_x;
     bool ok = true;
     uint32_t phase = 0;
     int issued = 0;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int ty = tile / tiles_x, x0 = (tile % tiles_x) * kTileM;
-        /* B: dY of the tile's 128 pixels */
-        for (int i = tid; i < kTileM * OG; i += 128) {
-            const int p = i / OG, og = i % OG, gx = x0 + p;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (gx < w) v = *reinterpret_cast<const uint4 *>(dy + ((size_t)ty * w + gx) * COUT + og * 8);
-            *reinterpret_cast<uint4 *>(sB + (p >> 3) * (OG * 128) + og * 128 + (p & 7) * 16) = v;
-        }
+        /* B: dY of the tile's 128 pixels, channel group tid % OG */
+        static_assert(kWgradThreads % OG == 0 && kTileM * OG <= kWgradThreads, "one load of B per thread");
+        uint4 bv = make_uint4(0, 0, 0, 0);
+        if (tid < kTileM * OG && x0 + tid / OG < w)
+            bv = *reinterpret_cast<const uint4 *>(dy + ((size_t)ty * w + x0 + tid / OG) * COUT + tid % OG * 8);
         /* A: the input at each tap's shift, zero outside the image */
-        for (int i = tid; i < NG * TG * CG * kTileM; i += 128) {
-            const int p = i % kTileM, rest = i / kTileM;
-            const int cg = rest % CG, slot = rest / CG; /* slot = g * TG + tl */
-            const int g = slot / TG, tl = slot % TG, t = slot;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (t < 9) {
-                const int gy = ty + t / 3 - 1, gx = x0 + p + t % 3 - 1;
-                if (x0 + p < w && gy >= 0 && gy < h && gx >= 0 && gx < w)
-                    v = *reinterpret_cast<const uint4 *>(x + ((size_t)gy * w + gx) * CIN + cg * 8);
+        constexpr int kALoads = NG * TG * CG * kTileM / kWgradThreads;
+        static_assert(NG * TG * CG * kTileM % kWgradThreads == 0 && kWgradThreads % kTileM == 0, "whole rounds of A");
+        uint4 av[kALoads];
+        const int p = tid % kTileM;
+#pragma unroll
+        for (int k = 0; k < kALoads; ++k) {
+            const int rest = tid / kTileM + k * (kWgradThreads / kTileM);
+            const int cg = rest % CG, t = rest / CG; /* t = g * TG + tl */
+            const int gy = ty + t / 3 - 1, gx = x0 + p + t % 3 - 1;
+            av[k] = make_uint4(0, 0, 0, 0);
+            if (t < 9 && x0 + p < w && gy >= 0 && gy < h && gx >= 0 && gx < w)
+                av[k] = *reinterpret_cast<const uint4 *>(x + ((size_t)gy * w + gx) * CIN + cg * 8);
+        }
+        if (tid < kTileM * OG) {
+            const int bp = tid / OG;
+            *reinterpret_cast<uint4 *>(sB + (bp >> 3) * (OG * 128) + tid % OG * 128 + (bp & 7) * 16) = bv;
+            const uint32_t v[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { /* BF16 is the upper half of the FP32 of the same value */
+                bsum[2 * c] += __uint_as_float(v[c] << 16);
+                bsum[2 * c + 1] += __uint_as_float(v[c] & 0xffff0000u);
             }
-            *reinterpret_cast<uint4 *>(sA + g * L::kAGroup + (p >> 3) * 2048 + (tl * CG + cg) * 128 + (p & 7) * 16) = v;
+        }
+#pragma unroll
+        for (int k = 0; k < kALoads; ++k) {
+            const int rest = tid / kTileM + k * (kWgradThreads / kTileM);
+            const int cg = rest % CG, t = rest / CG, g = t / TG, tl = t % TG;
+            *reinterpret_cast<uint4 *>(sA + g * L::kAGroup + (p >> 3) * 2048 + (tl * CG + cg) * 128 + (p & 7) * 16) = av[k];
         }
         tc::fence_proxy_async();
         tc::fence_before_sync();
@@ -292,18 +319,43 @@ __global__ void __launch_bounds__(128, 1)
         ok = __syncthreads_and(ok) != 0;
     }
     tc::fence_after_sync();
-    if (ok && issued) {
-        /* row m of group g: tap g * TG + m / CIN, input channel m % CIN */
-        const int m = warp * 32 + lane, tl = m / CIN, ci = m % CIN;
+    if (db && tid < kTileM * OG) {
+        /* lanes OG apart hold the same channels */
 #pragma unroll
-        for (int g = 0; g < NG; ++g) {
+        for (int c = 0; c < 8; ++c) {
+#pragma unroll
+            for (int o = 16; o >= OG; o >>= 1) bsum[c] += __shfl_xor_sync(0xffffffffu, bsum[c], o);
+            if (lane < OG) atomicAdd(&sDb[lane * 8 + c], bsum[c]);
+        }
+    }
+    __syncthreads();
+    if (db && tid < COUT) atomicAdd(&db[tid], sDb[tid]);
+    if (ok && issued) {
+        /* row m of group g: tap g * TG + m / CIN, input channel m % CIN; a
+         * warp reads the quarter of the TMEM lanes that its number gives it,
+         * and every fourth warp another group.  The sums go through shared
+         * memory (A's, whose MMAs are done) so that the atomics of a warp are
+         * one run of dW, and each CTA starts at another place of it: in TMEM
+         * order, all CTAs on the same scattered addresses at once, they took
+         * about half of the kernel's time. */
+        static_assert(NG <= kWgradThreads / 128, "a group per four warps");
+        constexpr int kDw = COUT * CIN * 9, kRounds = (kDw + kWgradThreads - 1) / kWgradThreads;
+        static_assert(kDw * 4 <= L::kA, "dW in A's memory");
+        float *sDw = reinterpret_cast<float *>(sA);
+        const int m = (warp & 3) * 32 + lane, tl = m / CIN, ci = m % CIN, g = warp >> 2;
+        if (g < NG) {
             uint32_t r[COUT];
-            load_acc<COUT>(tmem + g * COUT + ((uint32_t)(warp * 32) << 16), r);
+            load_acc<COUT>(tmem + g * COUT + ((uint32_t)((warp & 3) * 32) << 16), r);
             tc::tmem_wait_ld();
             const int t = g * TG + tl;
             if (t < 9)
 #pragma unroll
-                for (int n = 0; n < COUT; ++n) atomicAdd(&dw[((size_t)n * CIN + ci) * 9 + t], __uint_as_float(r[n]));
+                for (int n = 0; n < COUT; ++n) sDw[(n * CIN + ci) * 9 + t] = __uint_as_float(r[n]);
+        }
+        __syncthreads();
+        for (int k = 0; k < kRounds; ++k) {
+            const int e = (k + (int)(blockIdx.x % kRounds)) % kRounds * kWgradThreads + tid;
+            if (e < kDw) atomicAdd(&dw[e], sDw[e]);
         }
     } else if (!ok) {
         if (tid == 0) atomicExch(err, 1);
@@ -312,25 +364,6 @@ __global__ void __launch_bounds__(128, 1)
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 128);
-}
-
-/* Bias gradient db[c] += sum over pixels of dY[p][c] (dY FP32 or BF16). */
-template <typename T, int C>
-__global__ void k_bias_grad(const T *__restrict__ dy, long long n, float *__restrict__ db)
-{
-    float acc[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = 0.0f;
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
-#pragma unroll
-        for (int c = 0; c < C; ++c) acc[c] += (float)dy[p * C + c];
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-        float v = acc[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&db[c], v);
-    }
 }
 
 /* Weights [cout][cin][3][3] FP32 (PyTorch's OIHW) into the shared-memory
@@ -444,15 +477,15 @@ cudaError_t net_pack_weights(const float *wt, int cout, int cin, int mode, void 
     return cudaGetLastError();
 }
 
-cudaError_t net_conv_wgrad(const void *x, const void *dy, int h, int w, int cin, int cout, float *dw, int *err,
-                           int ctas, cudaStream_t s)
+cudaError_t net_conv_wgrad(const void *x, const void *dy, int h, int w, int cin, int cout, float *dw, float *db,
+                           int *err, int ctas, cudaStream_t s)
 {
     auto run = [&](auto kern, int bytes) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         const int tiles = h * ((w + kTileM - 1) / kTileM);
-        kern<<<tiles < ctas ? tiles : ctas, 128, bytes, s>>>(static_cast<const __nv_bfloat16 *>(x),
-                                                             static_cast<const __nv_bfloat16 *>(dy), h, w, dw, err);
+        kern<<<tiles < ctas ? tiles : ctas, kWgradThreads, bytes, s>>>(
+            static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dy), h, w, dw, db, err);
         return cudaGetLastError();
     };
     if (cin == 16 && cout == 32) return run(k_conv_wgrad<16, 32>, WgradSmem<16, 32>::kBytes);
@@ -460,20 +493,6 @@ cudaError_t net_conv_wgrad(const void *x, const void *dy, int h, int w, int cin,
     if (cin == 32 && cout == 16) return run(k_conv_wgrad<32, 16>, WgradSmem<32, 16>::kBytes);
     if (cin == 16 && cout == 16) return run(k_conv_wgrad<16, 16>, WgradSmem<16, 16>::kBytes);
     return cudaErrorInvalidValue;
-}
-
-cudaError_t net_bias_grad(const void *dy, int is_f32, long long n, int c, float *db, cudaStream_t s)
-{
-    const int blocks = 296;
-    if (is_f32 && c == 16) k_bias_grad<float, 16><<<blocks, 256, 0, s>>>(static_cast<const float *>(dy), n, db);
-    else if (is_f32 && c == 32) k_bias_grad<float, 32><<<blocks, 256, 0, s>>>(static_cast<const float *>(dy), n, db);
-    else if (!is_f32 && c == 16)
-        k_bias_grad<__nv_bfloat16, 16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(dy), n, db);
-    else if (!is_f32 && c == 32)
-        k_bias_grad<__nv_bfloat16, 32><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(dy), n, db);
-    else
-        return cudaErrorInvalidValue;
-    return cudaGetLastError();
 }
 
 }  // namespace hpm
@@ -514,7 +533,5 @@ extern "C" int hpm_net_conv_wgrad(const void *x, const void *dy, int h, int w, i
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (hpm::net_conv_wgrad(x, dy, h, w, cin, cout, dw, e, sms, s) != cudaSuccess) return HPM_ERR_CUDA;
-    if (db && hpm::net_bias_grad(dy, 0, (long long)h * w, cout, db, s) != cudaSuccess) return HPM_ERR_CUDA;
-    return HPM_OK;
+    return hpm::net_conv_wgrad(x, dy, h, w, cin, cout, dw, db, e, 2 * sms, s) == cudaSuccess ? HPM_OK : HPM_ERR_CUDA;
 }

@@ -13,8 +13,8 @@ namespace hpm {
 cudaError_t net_conv3x3(const void *x, int h, int w, int cin, const void *wpk, const float *bias, int cout, int epi,
                         const void *aux, void *y, int *err, bool use_tma, cudaStream_t s);
 cudaError_t net_pack_weights(const float *wt, int cout, int cin, int mode, void *out, cudaStream_t s);
-cudaError_t net_conv_wgrad(const void *x, const void *dy, int h, int w, int cin, int cout, float *dw, int *err,
-                           int ctas, cudaStream_t s);
-cudaError_t net_bias_grad(const void *dy, int is_f32, long long n, int c, float *db, cudaStream_t s);
+/* weight gradient, and the bias gradient where db is given */
+cudaError_t net_conv_wgrad(const void *x, const void *dy, int h, int w, int cin, int cout, float *dw, float *db,
+                           int *err, int ctas, cudaStream_t s);
 
 }  // namespace hpm
