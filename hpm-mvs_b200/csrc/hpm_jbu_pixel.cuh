@@ -15,6 +15,17 @@
  * per coarse pixel, so that every tap is a single 16-byte read-only load.
  * The reference computes both gaussians in double precision (pow/exp of a
  * double); here they are FP32 expf of the same arguments.
+ *
+ * What bounds it is the arithmetic of the (s*s+1)^2 taps (two expf each).  A
+ * tap whose coarse sample is more than sqrt(45) coarse pixels away has a
+ * spatial weight exp(-90) or less, which is zero in FP32, and adding zero
+ * changes no sum: at scale 4 these are 152 of the 289 taps.  They are left
+ * out where every value in reach of the block is finite (a weight of zero
+ * times an infinity is not zero); elsewhere all taps are taken.  Away from
+ * the borders, with a power of two as the scale, coordinates are exact and a
+ * row's taps are a plain run of the coarse grid, without conversions and
+ * clamps.  1600x1200 from 400x300: 775 us with all taps, 430 us now, the
+ * same bits.
  */
 #pragma once
 
@@ -22,49 +33,114 @@
 
 namespace hpm {
 
+constexpr int kJbuBlockX = 32, kJbuBlockY = 8;
+constexpr float kJbuReach2 = 45.0f; /* expf(-2 * 45) is 0 in FP32 */
+
+enum JbuTaps { kJbuAll, kJbuNear, kJbuInner };
+
+__device__ __forceinline__ int jbu_coarse(float v, int n)
+{
+    const int r = __float2int_rz(v);
+    return r > 0 ? (r < n ? r : n - 1) : 0;
+}
+
+/* How the block's pixels take their taps (the same answer in all threads; all
+ * must call). */
+__device__ __forceinline__ JbuTaps jbu_block_taps(const float *__restrict__ guide, int cols, int rows,
+                                                  const float4 *__restrict__ coarse, int s_cols, int s_rows,
+                                                  int image_scale)
+{
+    const float scale = (float)(1.0 * s_cols / cols);
+    const int nn = (image_scale * image_scale + 1) / 2;
+    const int x0 = blockIdx.x * kJbuBlockX, y0 = blockIdx.y * kJbuBlockY;
+    const int x1 = min(x0 + kJbuBlockX, cols) - 1, y1 = min(y0 + kJbuBlockY, rows) - 1;
+    const int tid = threadIdx.y * kJbuBlockX + threadIdx.x;
+    bool finite = true;
+    const int cx0 = jbu_coarse(x0 * scale - nn, s_cols), cx1 = jbu_coarse(x1 * scale + nn, s_cols);
+    const int cy0 = jbu_coarse(y0 * scale - nn, s_rows), cy1 = jbu_coarse(y1 * scale + nn, s_rows);
+    const int cw = cx1 - cx0 + 1, cn = cw * (cy1 - cy0 + 1);
+    for (int i = tid; i < cn; i += kJbuBlockX * kJbuBlockY) {
+        const float4 c = __ldg(coarse + (size_t)(cy0 + i / cw) * s_cols + cx0 + i % cw);
+        finite = finite && isfinite(c.x) && isfinite(c.y) && isfinite(c.z) && isfinite(c.w);
+    }
+    const int gx0 = max(x0 - nn, 0), gy0 = max(y0 - nn, 0);
+    const int gw = min(x1 + nn, cols - 1) - gx0 + 1, gn = gw * (min(y1 + nn, rows - 1) - gy0 + 1);
+    for (int i = tid; i < gn; i += kJbuBlockX * kJbuBlockY)
+        finite = finite && isfinite(__ldg(guide + (size_t)(gy0 + i / gw) * cols + gx0 + i % gw));
+    if (__syncthreads_or(!finite)) return kJbuAll;
+    const bool exact = (__float_as_uint(scale) & 0x7fffffu) == 0u && cols < (1 << 16) && rows < (1 << 16);
+    const bool inside = x0 * scale >= nn && y0 * scale >= nn && x1 * scale + nn < s_cols && y1 * scale + nn < s_rows &&
+                        x0 >= nn && y0 >= nn && x1 + nn < cols && y1 + nn < rows;
+    return exact && inside ? kJbuInner : kJbuNear;
+}
+
+struct JbuSums {
+    float nf, ctot, nx, ny, nz;
+    __device__ __forceinline__ void add(float4 c, float dis, float ref_pix, float nb)
+    {
+        const float inv_2sd2 = 1.0f / (2.0f * 0.5f * 0.5f);
+        const float inv_2sr2 = 1.0f / (2.0f * 25.5f * 25.5f);
+        const float sg = expf(-dis * inv_2sd2);
+        const float xp = fabsf(ref_pix - nb);
+        const float rg = expf(-(xp * xp) * inv_2sr2);
+        const float tg = sg * rg;
+        nf += tg;
+        ctot += c.w * tg;
+        nx += c.x * tg;
+        ny += c.y * tg;
+        nz += c.z * tg;
+    }
+};
+
 /* Returns (nx, ny, nz, depth) of fine pixel (px, py). */
 __device__ __forceinline__ float4 jbu_pixel(const float *__restrict__ guide, int cols, int rows,
                                             const float4 *__restrict__ coarse, int s_cols, int s_rows,
-                                            int image_scale, int px, int py)
+                                            int image_scale, int px, int py, JbuTaps taps)
 {
     const float scale = (float)(1.0 * s_cols / cols);
     const int nn = (image_scale * image_scale + 1) / 2;
     const float oy = py * scale, ox = px * scale;
     const float ref_pix = __ldg(guide + (size_t)py * cols + px);
-    const float inv_2sd2 = 1.0f / (2.0f * 0.5f * 0.5f);
-    const float inv_2sr2 = 1.0f / (2.0f * 25.5f * 25.5f);
-    float nf = 0.0f, ctot = 0.0f, nx = 0.0f, ny = 0.0f, nz = 0.0f;
-    for (int j = -nn; j <= nn; ++j) {
-        int ry = __float2int_rz(oy + (float)j);
-        ry = ry > 0 ? (ry < s_rows ? ry : s_rows - 1) : 0;
-        const int rys = min(max(py + j, 0), rows - 1);
-        const float dy = oy - (float)ry;
-        const float *grow = guide + (size_t)rys * cols;
-        for (int i = -nn; i <= nn; ++i) {
-            int rx = __float2int_rz(ox + (float)i);
-            rx = rx > 0 ? (rx < s_cols ? rx : s_cols - 1) : 0;
-            const float4 c = __ldg(coarse + (size_t)ry * s_cols + rx);
-            const int rxs = min(max(px + i, 0), cols - 1);
-            const float nb = __ldg(grow + rxs);
-            const float dx = ox - (float)rx;
-            const float dis = dx * dx + dy * dy;
-            const float sg = expf(-dis * inv_2sd2);
-            const float xp = fabsf(ref_pix - nb);
-            const float rg = expf(-(xp * xp) * inv_2sr2);
-            const float tg = sg * rg;
-            nf += tg;
-            ctot += c.w * tg;
-            nx += c.x * tg;
-            ny += c.y * tg;
-            nz += c.z * tg;
+    JbuSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (taps == kJbuInner) {
+        const int bx = __float2int_rz(ox), by = __float2int_rz(oy);
+        const float fx = ox - (float)bx, fy = oy - (float)by;
+        const int nj = min(nn, 7);
+        for (int j = -nj; j <= nj; ++j) {
+            const float dy = fy - (float)j;
+            /* the row's taps within reach, and at most one more at each end */
+            const int ni = min(nn, (int)sqrtf(fmaxf(kJbuReach2 - dy * dy, 0.0f)) + 1);
+            const float4 *crow = coarse + (size_t)(by + j) * s_cols + bx;
+            const float *grow = guide + (size_t)(py + j) * cols + px;
+#pragma unroll 4
+            for (int i = -ni; i <= ni; ++i) {
+                const float dx = fx - (float)i;
+                s.add(__ldg(crow + i), dx * dx + dy * dy, ref_pix, __ldg(grow + i));
+            }
+        }
+    } else {
+        for (int j = -nn; j <= nn; ++j) {
+            const int ry = jbu_coarse(oy + (float)j, s_rows);
+            const int rys = min(max(py + j, 0), rows - 1);
+            const float dy = oy - (float)ry;
+            if (taps == kJbuNear && dy * dy > kJbuReach2) continue;
+            const float *grow = guide + (size_t)rys * cols;
+            for (int i = -nn; i <= nn; ++i) {
+                const int rx = jbu_coarse(ox + (float)i, s_cols);
+                const float dx = ox - (float)rx;
+                const float dis = dx * dx + dy * dy;
+                if (taps == kJbuNear && dis > kJbuReach2) continue;
+                const int rxs = min(max(px + i, 0), cols - 1);
+                s.add(__ldg(coarse + (size_t)ry * s_cols + rx), dis, ref_pix, __ldg(grow + rxs));
+            }
         }
     }
-    float4 n = make_float4(nx / nf, ny / nf, nz / nf, 0.0f);
+    float4 n = make_float4(s.nx / s.nf, s.ny / s.nf, s.nz / s.nf, 0.0f);
     const float inv = rsqrtf(n.x * n.x + n.y * n.y + n.z * n.z);
     n.x *= inv;
     n.y *= inv;
     n.z *= inv;
-    n.w = ctot / nf;
+    n.w = s.ctot / s.nf;
     return n;
 }
 
