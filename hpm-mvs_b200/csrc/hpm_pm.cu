@@ -71,6 +71,12 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
 #ifndef HPM_P2_MIN_BLOCKS
 #define HPM_P2_MIN_BLOCKS 7
 #endif
+/* k_prop_select waits for loads (cost rows, source depths): 32 warps, although
+ * some registers spill (1600x1200, 10 sources, plain and geometric pass, by
+ * blocks per SM: 6 0.76 and 0.83 ms, 12 0.50 and 0.83, 16 0.47 and 0.71). */
+#ifndef HPM_P3_MIN_BLOCKS
+#define HPM_P3_MIN_BLOCKS 16
+#endif
 
 /* ------------------------------------------------------------------ */
 /* Philox4x32-10 (Salmon et al., SC'11), counter = (pixel, step, n/4, salt) */
@@ -701,23 +707,37 @@ __device__ __forceinline__ void project(const float *P, const HpmCamera &c, floa
 }
 
 /* ComputeGeomConsistencyCost (HPM.cu:483-508; capped at a.geom_max, 5 there
- * and 3 in ACMM.cu:494-519) */
-__device__ __noinline__ float geom_cost(const PMArgs &a, int v, float4 h, int px, int py)
+ * and 3 in ACMM.cu:494-519), in two halves, so that callers can have several
+ * source depths on their way before they use one: the world point of pixel
+ * (px, py) on plane h, its place in view v with the depth there, and the
+ * distance of that depth's reprojection. */
+__device__ __forceinline__ void geom_point(const PMArgs &a, float4 h, int px, int py, float *P)
 {
-    const HpmCamera &rc = a.cam[0], &sc = a.cam[v];
-    const float depth = depth_from_plane(rc, h, px, py);
-    float P[3], spt[2], sd;
-    world_point(rc, (float)px, (float)py, depth, P);
-    project(P, sc, spt, sd);
+    const float depth = depth_from_plane(a.cam[0], h, px, py);
+    world_point(a.cam[0], (float)px, (float)py, depth, P);
+}
+
+__device__ __forceinline__ float geom_source(const PMArgs &a, int v, const float *P, float *spt)
+{
+    float sd;
+    project(P, a.cam[v], spt, sd);
     const ViewDev &sv = a.view[v];
-    const float src_depth = texel(sv.depth, sv.w, sv.h, __float2int_rz(spt[0]), __float2int_rz(spt[1]));
-    if (a.counters) atomicAdd(&a.counters[1], 1ull);
+    return texel(sv.depth, sv.w, sv.h, __float2int_rz(spt[0]), __float2int_rz(spt[1]));
+}
+
+__device__ __forceinline__ float geom_distance(const PMArgs &a, int v, int px, int py, const float *spt, float src_depth)
+{
     if (src_depth == 0.0f) return a.geom_max;
     float Q[3], bpt[2], rd;
-    world_point(sc, spt[0], spt[1], src_depth, Q);
-    project(Q, rc, bpt, rd);
+    world_point(a.cam[v], spt[0], spt[1], src_depth, Q);
+    project(Q, a.cam[0], bpt, rd);
     const float dx = px - bpt[0], dy = py - bpt[1];
     return fminf(a.geom_max, sqrtf(dx * dx + dy * dy));
+}
+
+__device__ __forceinline__ void count_geom(const PMArgs &a, unsigned n)
+{
+    if (a.counters) atomicAdd(&a.counters[1], (unsigned long long)n);
 }
 
 /* ------------------------------------------------------------------ */
@@ -1285,27 +1305,60 @@ __device__ __forceinline__ void prop_select_body(const PMArgs &a, int iter, int 
                 vw_hi |= (unsigned long long)vw[v] << (4 * (v - 16));
         }
 
-    float fc[8];
+    /* candidates' costs, and the current hypothesis's (HPM.cu:1637-1650) from
+     * the cost-vector cache */
+    const float4 cur = a.planes[center];
+    float fc[8], cost_now = 0.0f;
+    if (a.geom) {
+        /* view by view, three planes' source depths on their way at a time;
+         * one plane after the other over all views the kernel waited for each
+         * (1600x1200, 10 sources: 2.05 against 0.71 ms) */
+        float P[9][3], f[9];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        float f = 0.0f;
-        float4 hk = make_float4(0, 0, 0, 1);
-        if (a.geom && FLAG(k)) hk = a.planes[pos[k]];
+        for (int k = 0; k < 9; ++k) {
+            geom_point(a, k < 8 && FLAG(k) ? a.planes[pos[k]] : cur, px, py, P[k]);
+            f[k] = 0.0f;
+        }
+#pragma unroll 1
+        for (int v = 0; v < S; ++v) {
+            const float w = view_weight(vw_lo, vw_hi, v);
+            if (!(w > 0.0f)) continue;
 #pragma unroll
-        for (int v = 0; v < SMAX; ++v) {
-            if (v < S && vw[v] > 0) {
-                if (a.geom) {
-                    if (FLAG(k))
-                        f += vw[v] * (ROWC(k, v) + 0.1f * geom_cost(a, v + 1, hk, px, py));
-                    else
-                        f += vw[v] * (ROWC(k, v) + 0.1f * 5.0f);
-                } else {
-                    f += vw[v] * ROWC(k, v);
+            for (int b = 0; b < 9; b += 3) {
+                float spt[3][2], d[3], row[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    d[i] = geom_source(a, v + 1, P[b + i], spt[i]);
+                    row[i] = b + i < 8 ? ROWC(b + i, v) : *cache_at(a, v, sl);
+                }
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const int k = b + i;
+                    const float g = geom_distance(a, v + 1, px, py, spt[i], d[i]);
+                    const float c = k == 8 ? __fmaf_rn(kGeomW, g, row[i])
+                                           : (FLAG(k) ? __fmaf_rn(0.1f, g, row[i]) : row[i] + 0.1f * 5.0f);
+                    f[k] = __fmaf_rn(w, c, f[k]);
                 }
             }
+            count_geom(a, __popc(flags) + 1);
         }
-        fc[k] = f / wn;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fc[k] = f[k] / wn;
+        cost_now = f[8];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float f = 0.0f;
+#pragma unroll
+            for (int v = 0; v < SMAX; ++v)
+                if (v < S && vw[v] > 0) f += vw[v] * ROWC(k, v);
+            fc[k] = f / wn;
+        }
+#pragma unroll
+        for (int v = 0; v < SMAX; ++v)
+            if (v < S && vw[v] > 0) cost_now += vw[v] * *cache_at(a, v, sl);
     }
+    cost_now /= wn;
     int min_idx = 0;
     {
         float m = fc[0];
@@ -1317,21 +1370,8 @@ __device__ __forceinline__ void prop_select_body(const PMArgs &a, int iter, int 
             }
     }
 
-    /* re-score of the current hypothesis (HPM.cu:1637-1650), from the cache */
-    const float4 cur = a.planes[center];
     float4 plane = cur;
     int best_row = -1; /* -1: the cached current hypothesis */
-    float cost_now = 0.0f;
-#pragma unroll
-    for (int v = 0; v < SMAX; ++v) {
-        if (v < S && vw[v] > 0) {
-            if (a.geom)
-                cost_now += vw[v] * (*cache_at(a, v, sl) + kGeomW * geom_cost(a, v + 1, plane, px, py));
-            else
-                cost_now += vw[v] * *cache_at(a, v, sl);
-        }
-    }
-    cost_now /= wn;
     float cost = cost_now;
     bool sel_new = false; /* the selected views change to the weighted ones */
     float depth_now = depth_from_plane(cam, plane, px, py);
@@ -1427,7 +1467,7 @@ __device__ __forceinline__ void prop_select_body(const PMArgs &a, int iter, int 
 }
 
 template <int SMAX, int WW, bool ACMM>
-__global__ void __launch_bounds__(kBlock) k_prop_select(const __grid_constant__ PMArgs a, int iter, int color)
+__global__ void __launch_bounds__(kBlock, HPM_P3_MIN_BLOCKS) k_prop_select(const __grid_constant__ PMArgs a, int iter, int color)
 {
     int px, py;
     half_step_pixel_at(blockIdx.x, blockIdx.y, WW, color, px, py);
@@ -1566,10 +1606,20 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, cons
                 const float w = __shfl_sync(kAll, weight, p);
                 const float4 h = items.cand[wv][i][p];
                 const int qx = patch.x(q), qy = patch.y(q);
+                /* the geometric term's source depth comes in under the window */
+                float spt[2], depth = 0.0f;
+                if (a.geom && need) {
+                    float P[3];
+                    geom_point(a, h, qx, qy, P);
+                    depth = geom_source(a, v + 1, P, spt);
+                }
                 float c = ncc_quad(a, v + 1, qx, qy, need, h, patch.win(q), st);
                 if (need) {
                     __stcs(&a.cand_costs[(size_t)((kRefineRow + i) * S + v) * sl.nh + hc], c);
-                    if (a.geom) c = __fmaf_rn(kGeomW, geom_cost(a, v + 1, h, qx, qy), c);
+                    if (a.geom) {
+                        c = __fmaf_rn(kGeomW, geom_distance(a, v + 1, qx, qy, spt, depth), c);
+                        count_geom(a, 1);
+                    }
                     items.cost[wv][i][p] = __fmaf_rn(w, c, items.cost[wv][i][p]);
                 }
             }
@@ -1760,7 +1810,14 @@ __global__ void k_geom_costs(const __grid_constant__ PMArgs a, const float4 *pla
     if (px >= a.W || py >= a.H) return;
     const int c = py * a.W + px;
     const int S = a.n - 1;
-    for (int v = 1; v < a.n; ++v) out[(size_t)c * S + v - 1] = geom_cost(a, v, planes[c], px, py);
+    float P[3];
+    geom_point(a, planes[c], px, py, P);
+    for (int v = 1; v < a.n; ++v) {
+        float spt[2];
+        const float d = geom_source(a, v, P, spt);
+        out[(size_t)c * S + v - 1] = geom_distance(a, v, px, py, spt, d);
+        count_geom(a, 1);
+    }
 }
 
 /* The 36 source samples of the NCC window of listed pixels, per source view
