@@ -146,6 +146,7 @@ PMArgs make_args(hpm_ctx *c)
         a.view[i].h = c->cams[i].height;
     }
     a.pair = c->d_pair;
+    memcpy(a.pairs, c->h_pair, sizeof(a.pairs));
     a.planes = c->d_planes;
     a.costs = c->d_costs;
     a.views = c->d_views;
@@ -332,6 +333,8 @@ int hpm_set_views(hpm_ctx *c, const float *const *images, const HpmCamera *cams,
     CK(cudaMemsetAsync(c->d_views, 0, sizeof(uint32_t) * n, c->stream), "state clear");
     PMArgs a = make_args(c);
     CK(launch_pair_geom(a, c->d_pair, c->stream), "pair geometry");
+    CK(cudaMemcpyAsync(c->h_pair, c->d_pair, sizeof(PairGeom) * num_images, cudaMemcpyDeviceToHost, c->stream),
+       "pair geometry");
     c->has_state = false;
     /* synchronous semantics for the caller's host buffers */
     CK(cudaStreamSynchronize(c->stream), "hpm_set_views");

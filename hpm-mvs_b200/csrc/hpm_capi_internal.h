@@ -82,6 +82,7 @@ struct hpm_ctx {
     size_t depth_cap[hpm::kMaxViews] = {0};
     bool has_depth = false;
     hpm::PairGeom *d_pair = nullptr;
+    hpm::PairGeom h_pair[hpm::kMaxViews]; /* its values, for the kernel arguments */
 
     float4 *d_planes = nullptr;
     float *d_costs = nullptr;

@@ -51,6 +51,7 @@ struct PMArgs {
     HpmCamera cam[kMaxViews];
     ViewDev view[kMaxViews];
     const PairGeom *pair; /* [n], entry 0 unused */
+    PairGeom pairs[kMaxViews]; /* the same by value: a uniform index reads it from the constant bank */
     float4 *planes;
     float *costs;
     uint32_t *views;

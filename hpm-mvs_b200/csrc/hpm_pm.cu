@@ -551,7 +551,7 @@ __device__ __forceinline__ float ncc_quad(const PMArgs &a, int v, int px, int py
     v = __shfl_sync(kAll, v, 0);
     const HpmCamera &sc = a.cam[v];
     float H[9];
-    homography(a.cam[0], sc, a.pair[v], h, H);
+    homography(a.cam[0], sc, a.pairs[v], h, H);
     const float fpx = (float)px, fpy = (float)py;
     const float2 pt = warp(H, fpx, fpy);
     /* the reference reaches 2 for a flat window after the taps */
@@ -569,8 +569,8 @@ __device__ __forceinline__ float ncc_quad(const PMArgs &a, int v, int px, int py
 #pragma unroll
         for (int e = 0; e < 9; ++e) G[e] = __shfl_sync(kAll, H[e], w, 4);
         const float gx = __shfl_sync(kAll, fpx, w, 4), gy = __shfl_sync(kAll, fpy, w, 4);
-#pragma unroll
-        for (int b = 0; b < 9; ++b) s[w][b] = 0.0f;
+        /* without a window to fetch the samples stay unset: only the lane
+         * that has none sums them */
         if ((quad >> w) & 1u) {
             /* lane l takes tap l ^ w of each block (bit 0: along x, bit 1:
              * along y), so that the hand-over below needs no select on the
@@ -907,63 +907,64 @@ __device__ __forceinline__ bool first_site_valid(int k, int r, int px, int py, i
  * the minimum with fix_quirks).
  * Polylines: start (+/-5|6) shifted 8r outward, then 7 zig-zag steps of 2
  * (HPM.cu:1346-1471). */
-__device__ int select_site(const PMArgs &a, int k, int r, int px, int py)
+__device__ __forceinline__ int select_site(const PMArgs &a, int k, int r, int px, int py)
 {
     const int W = a.W, H = a.H;
     const float *costs = a.costs;
+    /* all sites' costs are loaded before the first is compared */
+    int q[8];
+    float c[8];
+    bool in[8];
+    const int n = (k & 1) ? 5 : 8;
     if (k & 1) {
         const int dx = (k == 5) ? -1 : (k == 7 ? 1 : 0);
         const int dy = (k == 1) ? -1 : (k == 3 ? 1 : 0);
         const int off = 5 + 10 * r;
-        int best = (py + dy * off) * W + (px + dx * off);
-        float cmin = costs[best];
-        for (int i = 1; i < 5; ++i) {
-            bool ok;
-            switch (k) {
-            case 1: ok = py > 4 + 2 * i + 10 * r; break;
-            case 3: ok = py < H - 5 - 2 * i - 10 * r; break;
-            case 5: ok = px > 4 + 2 * i + 10 * r; break;
-            default: ok = px < W - 5 - 2 * i - 10 * r; break;
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            if (i > 0) {
+                switch (k) {
+                case 1: ok = ok && py > 4 + 2 * i + 10 * r; break;
+                case 3: ok = ok && py < H - 5 - 2 * i - 10 * r; break;
+                case 5: ok = ok && px > 4 + 2 * i + 10 * r; break;
+                default: ok = ok && px < W - 5 - 2 * i - 10 * r; break;
+                }
             }
-            if (!ok) break;
-            const int q = (py + dy * (off + 2 * i)) * W + (px + dx * (off + 2 * i));
-            const float cq = costs[q];
-            if ((k == 7 && !a.fix_quirks) ? (cmin < cq) : (cq < cmin)) {
-                cmin = cq;
-                best = q;
-            }
+            q[i] = (py + dy * (off + 2 * i)) * W + (px + dx * (off + 2 * i));
+            in[i] = ok;
+            c[i] = ok ? costs[q[i]] : 0.0f;
         }
-        return best;
-    }
-    int sx, sy, ex, ey, ox, oy; /* start, even step, odd step */
-    switch (k) {
-    case 0: sx = -5 - 8 * r; sy = -6 - 8 * r; ex = -2; ey = 0; ox = 0; oy = -2; break;
-    case 2: sx = 6 + 8 * r; sy = -5 - 8 * r; ex = 0; ey = -2; ox = 2; oy = 0; break;
-    case 4: sx = 5 + 8 * r; sy = 6 + 8 * r; ex = 2; ey = 0; ox = 0; oy = 2; break;
-    default: sx = -6 - 8 * r; sy = 5 + 8 * r; ex = 0; ey = 2; ox = -2; oy = 0; break;
-    }
-    int x = px + sx, y = py + sy;
-    int best = y * W + x;
-    float cmin = costs[best];
-    for (int i = 0; i < 7; ++i) {
-        if ((i & 1) == 0) {
-            x += ex;
-            y += ey;
-        } else {
-            x += ox;
-            y += oy;
+    } else {
+        int sx, sy, ex, ey, ox, oy; /* start, even step, odd step */
+        switch (k) {
+        case 0: sx = -5 - 8 * r; sy = -6 - 8 * r; ex = -2; ey = 0; ox = 0; oy = -2; break;
+        case 2: sx = 6 + 8 * r; sy = -5 - 8 * r; ex = 0; ey = -2; ox = 2; oy = 0; break;
+        case 4: sx = 5 + 8 * r; sy = 6 + 8 * r; ex = 2; ey = 0; ox = 0; oy = 2; break;
+        default: sx = -6 - 8 * r; sy = 5 + 8 * r; ex = 0; ey = 2; ox = -2; oy = 0; break;
         }
-        if (x >= 0 && x < W && y < H && y >= 0) {
-            const int q = y * W + x;
-            const float cq = costs[q];
-            if (cq < cmin) {
-                cmin = cq;
-                best = q;
+        int x = px + sx, y = py + sy;
+        bool ok = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i > 0) {
+                x += (i & 1) ? ex : ox;
+                y += (i & 1) ? ey : oy;
+                ok = ok && x >= 0 && x < W && y < H && y >= 0;
             }
-        } else {
-            break;
+            q[i] = y * W + x;
+            in[i] = ok;
+            c[i] = ok ? costs[q[i]] : 0.0f;
         }
     }
+    int best = q[0];
+    float cmin = c[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i)
+        if (i < n && in[i] && ((k == 7 && !a.fix_quirks) ? (cmin < c[i]) : (c[i] < cmin))) {
+            cmin = c[i];
+            best = q[i];
+        }
     return best;
 }
 
@@ -1022,28 +1023,48 @@ __device__ __forceinline__ float dir_cost(const PMArgs &a, uint32_t code, int k,
     return (a.fix_quirks || (k == 0 && v == 0)) ? 2.0f : 0.0f; /* fix_quirks: the intended {2, 2, ...} */
 }
 
-/* The windows that a warp still has to score, packed: lanes take them 32 at a
- * time whatever pixel they belong to, so that a pixel with few distinct
- * candidates leaves no idle lanes.  pos[k][lane]: the site of candidate k of
- * the warp's pixel `lane`; item: candidate << 5 | lane. */
+/* Shared memory of the direction kernel's block: the sites of each pixel's
+ * candidates, the statistics of its window, and the windows still to score,
+ * packed: lanes take them 32 at a time whatever pixel they belong to, so that
+ * a pixel with few distinct candidates leaves no idle lanes.  item: candidate
+ * << 6 | pixel of the block; judge: of direction 0's row, the costs below the
+ * three rounds' thresholds and those above 1.2, 8 bits each. */
 struct DirItems {
-    int pos[8][32];
-    uint8_t item[8 * 32];
+    int pos[8][kBlock];
+    RefStats stats[kBlock];
+    uint32_t judge[kBlock];
+    uint16_t item[kBlockY][8 * 32];
+    int count[kBlockY];
 };
+
+__device__ __forceinline__ uint32_t judge_cost(float c, const float *good)
+{
+    return (c < good[0] ? 1u : 0u) | (c < good[1] ? 1u << 8 : 0u) | (c < good[2] ? 1u << 16 : 0u) |
+           (c > 1.2f ? 1u << 24 : 0u);
+}
 
 template <int WW>
 __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const Patch<WW> &patch, DirItems &items)
 {
     const int W = a.W, H = a.H, S = a.n - 1;
-    const int lane = threadIdx.x, q0 = threadIdx.y * kBlockX;
+    const int lane = threadIdx.x, wv = threadIdx.y, q0 = wv * kBlockX;
     const int px = patch.x(q0 + lane), py = patch.y(q0 + lane);
     const bool act = px < W && py < a.rows_cov;
     /* lanes outside the image stay for the warp's windows, on a pixel inside */
     const int cx = min(px, W - 1), cy = min(py, H - 1);
     const int center = cy * W + cx;
     const Slot sl = slot_of(a, cx, cy);
-    const RefStats rs = ref_window(patch.win(q0 + lane));
     const float4 cur = a.planes[center];
+    items.stats[q0 + lane] = ref_window(patch.win(q0 + lane));
+    items.judge[q0 + lane] = 0;
+    /* JudgeExtend's threshold of each round, by one lane each */
+    float good[3];
+    {
+        const int r = min(lane, 2);
+        const float g = (float)(0.8 * exp(-iter * iter * (3 - r) / 90.0));
+#pragma unroll
+        for (int i = 0; i < 3; ++i) good[i] = __shfl_sync(kAll, g, i);
+    }
 
     int pos[8];
     uint32_t flags = 0;
@@ -1061,47 +1082,68 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
      * (dir_cost resolves the row on reading). */
     uint32_t code = kCodeAllNone; /* 4 bits per direction */
     uint32_t eval_mask = 0;
+    float4 plane[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
+        plane[k] = cur;
         if (!act || !first_site_valid(k, 0, px, py, W, H)) continue;
         flags |= 1u << k;
         pos[k] = select_site(a, k, 0, px, py);
-        items.pos[k][lane] = pos[k];
-        const float4 c = a.planes[pos[k]];
-        uint32_t src = same_plane(c, cur) ? kRowCache : kRowNone;
+        items.pos[k][q0 + lane] = pos[k];
+        plane[k] = a.planes[pos[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (!((flags >> k) & 1u)) continue;
+        uint32_t src = same_plane(plane[k], cur) ? kRowCache : kRowNone;
 #pragma unroll
         for (int j = 0; j < k; ++j)
-            if (src == kRowNone && ((flags >> j) & 1u) && same_plane(c, a.planes[pos[j]])) src = (uint32_t)j;
+            if (src == kRowNone && ((flags >> j) & 1u) && same_plane(plane[k], plane[j])) src = (uint32_t)j;
         if (src == kRowNone) {
             src = kRowOwn;
             eval_mask |= 1u << k;
         }
         code = (code & ~(15u << (4 * k))) | (src << (4 * k));
     }
+    /* direction 0's row, where it is not scored here: judged on the spot */
+    auto judge_row = [&](uint32_t src) {
+        const float *row = src == kRowCache ? cache_at(a, 0, sl) : &CAG(src, 0);
+        const size_t stride = src == kRowCache ? 2 * sl.nh : sl.nh;
+        uint32_t sum = 0;
+#pragma unroll 5
+        for (int v = 0; v < S; ++v) sum += judge_cost(row[(size_t)v * stride], good);
+        items.judge[q0 + lane] = sum;
+    };
+    if ((code & 15u) == kRowCache) judge_row(kRowCache);
     /* 2) the distinct candidates, view by view, so that the threads of a
      * block sample one source image at a time (texture-cache locality).
      * Round 0 scores the sites; rounds 1 to 3 are the extension.
      * Extension: only the left-up polyline can extend, because
      * bool symbol_eight_orientations[10] = { true } sets index 0 only
-     * (HPM.cu:1475).  JudgeExtend: HPM.cu:1036-1059. */
+     * (HPM.cu:1475).  JudgeExtend: HPM.cu:1036-1059, from counts kept while
+     * the row is scored.  The extension has few windows a view, so both warps'
+     * are packed together and the views dealt out to the warps. */
     bool extend = (flags & 1u) != 0;
     bool detached = false; /* rows that copy direction 0's first row hold their own copy */
 #pragma unroll 1
     for (int round = 0; round < 4; ++round) {
-        if (round > 0) {
+        int total = 0;
+        if (round == 0) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const bool mine = (eval_mask >> k) & 1u;
+                const unsigned m = __ballot_sync(kAll, mine);
+                if (mine) items.item[wv][total + __popc(m & lanes_below())] = (uint16_t)(k << 6 | (q0 + lane));
+                total += __popc(m);
+            }
+            __syncwarp();
+        } else {
             const int r = round - 1;
-            eval_mask = 0;
-            if (!__any_sync(kAll, extend)) break;
-            __syncwarp(); /* the rows scored by other lanes */
-            const float good = (float)(0.8 * exp(-iter * iter * (3 - r) / 90.0));
+            bool mine = false;
+            if (!__syncthreads_or(extend)) break; /* also: the rows and counts of the last round are there */
             if (extend) {
-                int good_sum = 0, bad_sum = 0;
-                for (int v = 0; v < S; ++v) {
-                    const float c = dir_cost(a, code, 0, v, S, sl);
-                    if (c < good) good_sum++;
-                    if (c > 1.2f) bad_sum++;
-                }
-                if (good_sum >= 1 && bad_sum <= 2) extend = false;
+                const uint32_t counts = items.judge[q0 + lane];
+                if (((counts >> (8 * r)) & 255u) >= 1u && (counts >> 24) <= 2u) extend = false;
             }
             /* an invalid first site keeps site and costs: flag[0] is set */
             if (extend && first_site_valid(0, r, px, py, W, H)) {
@@ -1109,9 +1151,9 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
                 /* a better previous site is kept */
                 if (!(a.costs[best] > a.costs[pos[0]])) {
                     const float4 prev = a.planes[pos[0]];
-                    pos[0] = best;
-                    items.pos[0][lane] = best;
                     const float4 p = a.planes[best];
+                    pos[0] = best;
+                    items.pos[0][q0 + lane] = best;
                     if (!same_plane(p, prev)) {
                         /* direction 0's row changes: the rows that refer to
                          * it keep the values it had when they were chosen */
@@ -1124,46 +1166,57 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
                                     code = (code & ~(15u << (4 * k))) | (kRowOwn << (4 * k));
                                 }
                         }
+                        float first[8]; /* loaded together; equal planes have equal first components */
+#pragma unroll
+                        for (int j = 1; j < 8; ++j) first[j] = ((flags >> j) & 1u) ? a.planes[pos[j]].x : 0.0f;
                         int src = -1;
 #pragma unroll
                         for (int j = 1; j < 8; ++j)
-                            if (src < 0 && ((flags >> j) & 1u) && same_plane(p, a.planes[pos[j]])) src = j;
+                            if (src < 0 && ((flags >> j) & 1u) && __float_as_uint(first[j]) == __float_as_uint(p.x) &&
+                                same_plane(p, a.planes[pos[j]]))
+                                src = j;
                         if (same_plane(p, cur)) {
                             code = (code & ~15u) | kRowCache;
+                            judge_row(kRowCache);
                         } else if (src >= 0) {
-                            const uint32_t sj = (code >> (4 * src)) & 15u;
-                            code = (code & ~15u) | (sj == kRowOwn ? (uint32_t)src : sj);
+                            const uint32_t sj = (code >> (4 * src)) & 15u, at = sj == kRowOwn ? (uint32_t)src : sj;
+                            code = (code & ~15u) | at;
+                            judge_row(at);
                         } else {
-                            eval_mask = 1u;
+                            mine = true;
                             code = (code & ~15u) | kRowOwn;
+                            items.judge[q0 + lane] = 0;
                         }
                     }
                 }
             }
+            eval_mask = mine ? 1u : 0u;
+            const unsigned m = __ballot_sync(kAll, mine);
+            if (lane == 0) items.count[wv] = __popc(m);
+            __syncthreads();
+            if (mine) items.item[0][(wv ? items.count[0] : 0) + __popc(m & lanes_below())] = (uint16_t)(q0 + lane);
+            total = items.count[0] + items.count[1];
+            __syncthreads();
         }
-        int total = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const unsigned m = __ballot_sync(kAll, (eval_mask >> k) & 1u);
-            if ((eval_mask >> k) & 1u) items.item[total + __popc(m & lanes_below())] = (uint8_t)(k << 5 | lane);
-            total += __popc(m);
-        }
-        __syncwarp();
+        const uint16_t *list = items.item[round == 0 ? wv : 0];
+        const int step = round == 0 ? 1 : kBlockY;
 #pragma unroll 1
-        for (int v = 0; v < S; ++v)
+        for (int v = round == 0 ? 0 : wv; v < S; v += step)
 #pragma unroll 1
             for (int base = 0; base < total; base += 32) {
                 const bool need = base + lane < total;
-                const int it = items.item[need ? base + lane : 0], k = it >> 5, p = it & 31, q = q0 + p;
-                const RefStats st = stats_of(rs, p);
-                const int hc = __shfl_sync(kAll, sl.hc, p);
-                const float c = ncc_quad(a, v + 1, patch.x(q), patch.y(q), need, a.planes[items.pos[k][p]],
-                                         patch.win(q), st);
-                if (need) __stcs(&a.cand_costs[(size_t)(k * S + v) * sl.nh + hc], c);
+                const int it = list[need ? base + lane : 0], k = it >> 6, q = it & 63;
+                const RefStats st = items.stats[q];
+                const int qx = patch.x(q), qy = patch.y(q);
+                const float c = ncc_quad(a, v + 1, qx, qy, need, a.planes[need ? items.pos[k][q] : center], patch.win(q), st);
+                if (need) {
+                    __stcs(&a.cand_costs[(size_t)(k * S + v) * sl.nh + ((qy * W + qx) >> 1)], c);
+                    if (k == 0) atomicAdd(&items.judge[q], judge_cost(c, good));
+                }
             }
         if (a.counters && eval_mask) atomicAdd(&a.counters[0], (unsigned long long)(__popc(eval_mask) * S));
     }
-    __syncwarp();
+    __syncthreads();
     if (!act) return;
     /* 3) every valid direction's row in its own slot: a row that refers to
      * the cost-vector cache or to an earlier direction (always one that owns
@@ -1188,8 +1241,8 @@ __global__ void __launch_bounds__(kBlock, HPM_P1_MIN_BLOCKS) k_prop_dirs(const _
                                                                           int color)
 {
     __shared__ PatchMem<WW> sPatch;
-    __shared__ DirItems sItems[kBlockY];
-    prop_dirs_body(a, iter, sPatch.load(a, color), sItems[threadIdx.y]);
+    __shared__ DirItems sItems;
+    prop_dirs_body(a, iter, sPatch.load(a, color), sItems);
 }
 
 /* What the selection hands to the refinement, per pixel (rf_* in PMArgs):
