@@ -138,6 +138,7 @@ extern "C" int hpm_run_scene_acmm(hpm_ctx *c, int n_views, const float *const *i
     CK(ctx_scene_arena(c, total * sizeof(float)), "scene buffers");
     float *base = ctx_scene_base(c);
     std::vector<float *> full(n_views);
+    std::vector<CopyItem> copies;
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)cams[v].width * cams[v].height, sp = st(np);
         full[v] = base;
@@ -147,8 +148,9 @@ extern "C" int hpm_run_scene_acmm(hpm_ctx *c, int n_views, const float *const *i
         m.normal.push_back(base + 4 * sp);
         m.cost.push_back(base + 7 * sp);
         base += 8 * sp;
-        CK(cudaMemcpyAsync(full[v], images[v], sizeof(float) * np, cudaMemcpyDefault, s), "scene images");
+        copies.push_back({full[v], images[v], sizeof(float) * np});
     }
+    CK(ctx_copy_in(c, copies.data(), n_views), "scene images");
     m.coarse = reinterpret_cast<float4 *>(base);
     m.up_normal = reinterpret_cast<float4 *>(base + 4 * st(largest));
     m.up_depth = base + 8 * st(largest);
@@ -278,16 +280,14 @@ extern "C" int hpm_run_scene_acmm(hpm_ctx *c, int n_views, const float *const *i
                 if ((r = geometric(p, gi > 0))) return r;
         max_down--;
     }
+    copies.clear();
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)m.at[v].w * m.at[v].h;
         const float *d = o->geom_iterations > 0 ? m.depth_g[v] : m.depth[v];
-        if (out_depths && out_depths[v])
-            CK(cudaMemcpyAsync(out_depths[v], d, sizeof(float) * np, cudaMemcpyDefault, s), "out");
-        if (out_normals && out_normals[v])
-            CK(cudaMemcpyAsync(out_normals[v], m.normal[v], sizeof(float) * 3 * np, cudaMemcpyDefault, s), "out");
-        if (out_costs && out_costs[v])
-            CK(cudaMemcpyAsync(out_costs[v], m.cost[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
+        if (out_depths && out_depths[v]) copies.push_back({out_depths[v], d, sizeof(float) * np});
+        if (out_normals && out_normals[v]) copies.push_back({out_normals[v], m.normal[v], sizeof(float) * 3 * np});
+        if (out_costs && out_costs[v]) copies.push_back({out_costs[v], m.cost[v], sizeof(float) * np});
     }
-    CK(cudaStreamSynchronize(s), "hpm_run_scene_acmm");
+    CK(ctx_copy_out(c, copies.data(), (int)copies.size()), "hpm_run_scene_acmm");
     return HPM_OK;
 }

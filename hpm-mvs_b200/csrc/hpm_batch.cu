@@ -345,6 +345,7 @@ int batched_scene(hpm_ctx *c, int n_views, const float *const *images, const Hpm
     for (int v = 0; v < n_views; ++v) total += 8 * (((size_t)cams[v].width * cams[v].height + 63) & ~(size_t)63);
     CK(ctx_scene_arena(c, total * sizeof(float)), "scene buffers");
     float *cur = ctx_scene_base(c);
+    std::vector<CopyItem> copies;
     CK(cudaMemsetAsync(cur, 0, total * sizeof(float), s), "scene buffers");
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)cams[v].width * cams[v].height, st = (np + 63) & ~(size_t)63;
@@ -355,8 +356,9 @@ int batched_scene(hpm_ctx *c, int n_views, const float *const *images, const Hpm
         nrm[v] = cur + 4 * st;
         cst[v] = cur + 7 * st;
         cur += 8 * st;
-        CK(cudaMemcpyAsync(img[v], images[v], sizeof(float) * np, cudaMemcpyDefault, s), "scene images");
+        copies.push_back({img[v], images[v], sizeof(float) * np});
     }
+    CK(ctx_copy_in(c, copies.data(), n_views), "scene images");
     CK(cudaStreamSynchronize(s), "scene images");
     /* one context per problem, kept for later scenes */
     while ((int)c->batch.size() < n_problems) {
@@ -503,16 +505,14 @@ int batched_scene(hpm_ctx *c, int n_views, const float *const *images, const Hpm
         src = dst;
         dst = (dst == &dep_g0) ? &dep_g1 : &dep_g0;
     }
+    copies.clear();
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)cams[v].width * cams[v].height;
-        if (out_depths && out_depths[v])
-            CK(cudaMemcpyAsync(out_depths[v], (*src)[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
-        if (out_normals && out_normals[v])
-            CK(cudaMemcpyAsync(out_normals[v], nrm[v], sizeof(float) * 3 * np, cudaMemcpyDefault, s), "out");
-        if (out_costs && out_costs[v])
-            CK(cudaMemcpyAsync(out_costs[v], cst[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
+        if (out_depths && out_depths[v]) copies.push_back({out_depths[v], (*src)[v], sizeof(float) * np});
+        if (out_normals && out_normals[v]) copies.push_back({out_normals[v], nrm[v], sizeof(float) * 3 * np});
+        if (out_costs && out_costs[v]) copies.push_back({out_costs[v], cst[v], sizeof(float) * np});
     }
-    CK(cudaStreamSynchronize(s), "hpm_run_scene_batched");
+    CK(ctx_copy_out(c, copies.data(), (int)copies.size()), "hpm_run_scene_batched");
     return HPM_OK;
 }
 

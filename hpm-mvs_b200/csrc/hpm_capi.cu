@@ -257,6 +257,7 @@ int hpm_destroy(hpm_ctx *c)
     cudaFree(c->d_flags);
     cudaFree(c->d_refine);
     cudaFree(c->d_pre);
+    host_copier_free(c->copier);
     ws_free(c);
     net_free(c);
     for (auto &p : c->prof_events) {
@@ -286,10 +287,14 @@ int hpm_set_views(hpm_ctx *c, const float *const *images, const HpmCamera *cams,
     }
     int r = select_device(c);
     if (r) return r;
+    CopyItem items[kMaxViews];
     for (int i = 0; i < num_images; ++i) {
         const size_t bytes = sizeof(float) * cams[i].width * cams[i].height;
         CK(ensure((void **)&c->d_img[i], &c->img_cap[i], bytes), "image alloc");
-        CK(cudaMemcpyAsync(c->d_img[i], images[i], bytes, cudaMemcpyDefault, c->stream), "image upload");
+        items[i] = {c->d_img[i], images[i], bytes};
+    }
+    CK(ctx_copy_in(c, items, num_images), "image upload");
+    for (int i = 0; i < num_images; ++i) {
         CK(ensure_texture(c, i, cams[i].width, cams[i].height), "texture set-up");
         CK(cudaMemcpy2DToArrayAsync(c->arr[i], 0, 0, c->d_img[i], sizeof(float) * cams[i].width,
                                     sizeof(float) * cams[i].width, cams[i].height, cudaMemcpyDeviceToDevice,
@@ -348,12 +353,14 @@ int hpm_set_geom_depths(hpm_ctx *c, const float *const *depths)
     if (!depths) return fail(c, HPM_ERR_ARG, "hpm_set_geom_depths: null");
     int r = select_device(c);
     if (r) return r;
+    CopyItem items[kMaxViews];
     for (int i = 0; i < c->n; ++i) {
         if (!depths[i]) return fail(c, HPM_ERR_ARG, "hpm_set_geom_depths: depth %d is null", i);
         const size_t bytes = sizeof(float) * c->cams[i].width * c->cams[i].height;
         CK(ensure((void **)&c->d_depth[i], &c->depth_cap[i], bytes), "depth alloc");
-        CK(cudaMemcpyAsync(c->d_depth[i], depths[i], bytes, cudaMemcpyDefault, c->stream), "depth upload");
+        items[i] = {c->d_depth[i], depths[i], bytes};
     }
+    CK(ctx_copy_in(c, items, c->n), "depth upload");
     c->has_depth = true;
     CK(cudaStreamSynchronize(c->stream), "hpm_set_geom_depths");
     return HPM_OK;
@@ -367,10 +374,9 @@ int hpm_set_hypotheses(hpm_ctx *c, const float *planes, const float *costs)
     int r = select_device(c);
     if (r) return r;
     const size_t n = npx(c);
-    CK(cudaMemcpyAsync(c->d_planes, planes, sizeof(float4) * n, cudaMemcpyDefault, c->stream), "planes");
-    if (costs)
-        CK(cudaMemcpyAsync(c->d_costs, costs, sizeof(float) * n, cudaMemcpyDefault, c->stream), "costs");
-    else
+    const CopyItem items[2] = {{c->d_planes, planes, sizeof(float4) * n}, {c->d_costs, costs, sizeof(float) * n}};
+    CK(ctx_copy_in(c, items, costs ? 2 : 1), "hypotheses");
+    if (!costs)
         CK(cudaMemsetAsync(c->d_costs, 0, sizeof(float) * n, c->stream), "costs");
     c->has_state = true;
     CK(cudaStreamSynchronize(c->stream), "hpm_set_hypotheses");
@@ -385,8 +391,8 @@ int hpm_set_prior(hpm_ctx *c, const float *prior_planes, const uint32_t *masks)
     int r = select_device(c);
     if (r) return r;
     const size_t n = npx(c);
-    CK(cudaMemcpyAsync(c->d_prior, prior_planes, sizeof(float4) * n, cudaMemcpyDefault, c->stream), "prior");
-    CK(cudaMemcpyAsync(c->d_masks, masks, sizeof(uint32_t) * n, cudaMemcpyDefault, c->stream), "masks");
+    const CopyItem items[2] = {{c->d_prior, prior_planes, sizeof(float4) * n}, {c->d_masks, masks, sizeof(uint32_t) * n}};
+    CK(ctx_copy_in(c, items, 2), "prior");
     c->has_prior = true;
     CK(cudaStreamSynchronize(c->stream), "hpm_set_prior");
     return HPM_OK;
@@ -513,10 +519,11 @@ int hpm_get_result(hpm_ctx *c, float *planes, float *costs)
     int r = select_device(c);
     if (r) return r;
     const size_t n = npx(c);
-    if (planes)
-        CK(cudaMemcpyAsync(planes, c->d_planes, sizeof(float4) * n, cudaMemcpyDeviceToHost, c->stream), "planes");
-    if (costs) CK(cudaMemcpyAsync(costs, c->d_costs, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream), "costs");
-    CK(cudaStreamSynchronize(c->stream), "hpm_get_result");
+    CopyItem items[2];
+    int k = 0;
+    if (planes) items[k++] = {planes, c->d_planes, sizeof(float4) * n};
+    if (costs) items[k++] = {costs, c->d_costs, sizeof(float) * n};
+    CK(ctx_copy_out(c, items, k), "hpm_get_result");
     return HPM_OK;
 }
 
@@ -526,8 +533,8 @@ int hpm_get_selected_views(hpm_ctx *c, uint32_t *views)
     if (c->n < 2) return fail(c, HPM_ERR_STATE, "hpm_get_selected_views before hpm_set_views");
     int r = select_device(c);
     if (r) return r;
-    CK(cudaMemcpyAsync(views, c->d_views, sizeof(uint32_t) * npx(c), cudaMemcpyDeviceToHost, c->stream), "views");
-    CK(cudaStreamSynchronize(c->stream), "hpm_get_selected_views");
+    const CopyItem item = {views, c->d_views, sizeof(uint32_t) * npx(c)};
+    CK(ctx_copy_out(c, &item, 1), "hpm_get_selected_views");
     return HPM_OK;
 }
 

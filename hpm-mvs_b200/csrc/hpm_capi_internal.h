@@ -11,6 +11,7 @@
 #include <utility>
 #include <vector>
 
+#include "hpm_copy.h"
 #include "hpm_internal.h"
 
 namespace hpm {
@@ -131,6 +132,7 @@ struct hpm_ctx {
     std::vector<hpm_ctx *> batch;
     std::vector<std::pair<long long, int>> tile_ww;
     hpm::FlowWorkspace flow;
+    hpm::HostCopier *copier = nullptr; /* pinned buffers of ctx_copy_in / ctx_copy_out */
     /* HpmProblemOpts.fix_quirks of the problem being processed (prior levels) */
     bool fix_quirks = false;
     float *d_scene = nullptr; /* hpm_run_scene's per-view maps, grown on demand */

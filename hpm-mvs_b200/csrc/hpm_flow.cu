@@ -275,13 +275,14 @@ static int process_problem(hpm_ctx *c, const HpmProblemOpts *o, int half_steps, 
     k_split_state<<<grid1((int)npx), 256, 0, s>>>(reinterpret_cast<const float4 *>(ctx_planes(c)), (int)npx,
                                                   ws.full_depth, ws.full_normal);
     /* outputs may be host or device memory (unified addressing) */
-    if (depth_out) CK(cudaMemcpyAsync(depth_out, ws.full_depth, sizeof(float) * npx, cudaMemcpyDefault, s), "out");
-    if (normal_out)
-        CK(cudaMemcpyAsync(normal_out, ws.full_normal, sizeof(float) * 3 * npx, cudaMemcpyDefault, s), "out");
-    if (cost_out) CK(cudaMemcpyAsync(cost_out, ctx_costs(c), sizeof(float) * npx, cudaMemcpyDefault, s), "out");
+    CopyItem items[4];
+    int k = 0;
+    if (depth_out) items[k++] = {depth_out, ws.full_depth, sizeof(float) * npx};
+    if (normal_out) items[k++] = {normal_out, ws.full_normal, sizeof(float) * 3 * npx};
+    if (cost_out) items[k++] = {cost_out, ctx_costs(c), sizeof(float) * npx};
     if (prior_depth_out) {
         if (ws.has_prior_depth && o->planar_prior && !o->geom_consistency) {
-            CK(cudaMemcpyAsync(prior_depth_out, ws.prior_depth, sizeof(float) * npx, cudaMemcpyDefault, s), "out");
+            items[k++] = {prior_depth_out, ws.prior_depth, sizeof(float) * npx};
         } else {
             cudaPointerAttributes pa;
             if (cudaPointerGetAttributes(&pa, prior_depth_out) == cudaSuccess && pa.type == cudaMemoryTypeDevice)
@@ -290,7 +291,7 @@ static int process_problem(hpm_ctx *c, const HpmProblemOpts *o, int half_steps, 
                 memset(prior_depth_out, 0, sizeof(float) * npx);
         }
     }
-    CK(cudaStreamSynchronize(s), "hpm_process_problem");
+    CK(ctx_copy_out(c, items, k), "hpm_process_problem");
     return HPM_OK;
 }
 
@@ -394,6 +395,7 @@ static int run_scene_impl(hpm_ctx *c, int n_views, const float *const *images, c
     for (int v = 0; v < n_views; ++v) total += 7 * (((size_t)cams[v].width * cams[v].height + 63) & ~(size_t)63);
     CK(ctx_scene_arena(c, total * sizeof(float)), "scene buffers");
     float *cur = ctx_scene_base(c);
+    std::vector<CopyItem> copies;
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)cams[v].width * cams[v].height, st = (np + 63) & ~(size_t)63;
         m.img.push_back(cur);
@@ -402,8 +404,9 @@ static int run_scene_impl(hpm_ctx *c, int n_views, const float *const *images, c
         m.normal.push_back(cur + 3 * st);
         m.cost.push_back(cur + 6 * st);
         cur += 7 * st;
-        CK(cudaMemcpyAsync(m.img[v], images[v], sizeof(float) * np, cudaMemcpyDefault, s), "scene images");
+        copies.push_back({m.img[v], images[v], sizeof(float) * np});
     }
+    CK(ctx_copy_in(c, copies.data(), n_views), "scene images");
     /* the views of problem p */
     auto gather = [&](int p, const float **pimg, HpmCamera *pcam) -> int {
         const int ref = ref_ids[p], ns = src_counts[p];
@@ -517,17 +520,15 @@ static int run_scene_impl(hpm_ctx *c, int n_views, const float *const *images, c
         }
     }
     std::vector<float *> &final_depth = o->geom_iterations > 0 ? m.depth_g : m.depth_a;
+    copies.clear();
     for (int v = 0; v < n_views; ++v) {
         const size_t np = (size_t)cams[v].width * cams[v].height;
-        if (out_depths && out_depths[v])
-            CK(cudaMemcpyAsync(out_depths[v], final_depth[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
-        if (out_normals && out_normals[v])
-            CK(cudaMemcpyAsync(out_normals[v], m.normal[v], sizeof(float) * 3 * np, cudaMemcpyDefault, s), "out");
-        if (out_costs && out_costs[v])
-            CK(cudaMemcpyAsync(out_costs[v], m.cost[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
+        if (out_depths && out_depths[v]) copies.push_back({out_depths[v], final_depth[v], sizeof(float) * np});
+        if (out_normals && out_normals[v]) copies.push_back({out_normals[v], m.normal[v], sizeof(float) * 3 * np});
+        if (out_costs && out_costs[v]) copies.push_back({out_costs[v], m.cost[v], sizeof(float) * np});
         if (out_pass_depths && out_pass_depths[v])
-            CK(cudaMemcpyAsync(out_pass_depths[v], m.depth_a[v], sizeof(float) * np, cudaMemcpyDefault, s), "out");
+            copies.push_back({out_pass_depths[v], m.depth_a[v], sizeof(float) * np});
     }
-    CK(cudaStreamSynchronize(s), "hpm_run_scene");
+    CK(ctx_copy_out(c, copies.data(), (int)copies.size()), "hpm_run_scene");
     return HPM_OK;
 }
