@@ -74,6 +74,8 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
 /* k_prop_select waits for loads (cost rows, source depths): 32 warps, although
  * some registers spill (1600x1200, 10 sources, plain and geometric pass, by
  * blocks per SM: 6 0.76 and 0.83 ms, 12 0.50 and 0.83, 16 0.47 and 0.71). */
+/* and of their wide forms for small images (kBlocks8) */
+constexpr int kWideWarps = 16;
 #ifndef HPM_P3_MIN_BLOCKS
 #define HPM_P3_MIN_BLOCKS 16
 #endif
@@ -284,11 +286,12 @@ struct PatchMem {
     Spatial sp;
 
     /* fills the tile (all threads; edges repeated) and the spatial terms */
+    template <int NW>
     __device__ __forceinline__ Patch<WW> load(const PMArgs &a, int color)
     {
         const ViewDev &rv = a.view[0];
         const int x0 = (int)blockIdx.x * 2 * WW, y0 = (int)blockIdx.y * 2 * (32 / WW);
-        for (int i = threadIdx.y * kBlockX + threadIdx.x; i < Tile::kRows * Tile::kCols; i += kBlock) {
+        for (int i = threadIdx.y * kBlockX + threadIdx.x; i < Tile::kRows * Tile::kCols; i += kBlockX * NW) {
             const int r = i / Tile::kCols, c = i - r * Tile::kCols, ty = y0 - 5 + r;
             tile[r * Tile::kPitch + c] = texel(rv.img, rv.w, rv.h, x0 + ((ty + 1 + color) & 1) - 5 + 2 * c, ty);
         }
@@ -1043,20 +1046,24 @@ __device__ __forceinline__ uint32_t judge_cost(float c, const float *good)
            (c > 1.2f ? 1u << 24 : 0u);
 }
 
-template <int WW>
+template <int WW, int NW>
 __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const Patch<WW> &patch, DirItems &items)
 {
     const int W = a.W, H = a.H, S = a.n - 1;
-    const int lane = threadIdx.x, wv = threadIdx.y, q0 = wv * kBlockX;
+    /* the first two warps own the block's pixels, others only score */
+    const int lane = threadIdx.x, wv = threadIdx.y, q0 = (wv & 1) * kBlockX;
+    const bool owner = NW == kBlockY || wv < kBlockY;
     const int px = patch.x(q0 + lane), py = patch.y(q0 + lane);
-    const bool act = px < W && py < a.rows_cov;
+    const bool act = owner && px < W && py < a.rows_cov;
     /* lanes outside the image stay for the warp's windows, on a pixel inside */
     const int cx = min(px, W - 1), cy = min(py, H - 1);
     const int center = cy * W + cx;
     const Slot sl = slot_of(a, cx, cy);
     const float4 cur = a.planes[center];
-    items.stats[q0 + lane] = ref_window(patch.win(q0 + lane));
-    items.judge[q0 + lane] = 0;
+    if (owner) {
+        items.stats[q0 + lane] = ref_window(patch.win(q0 + lane));
+        items.judge[q0 + lane] = 0;
+    }
     /* JudgeExtend's threshold of each round, by one lane each */
     float good[3];
     {
@@ -1133,10 +1140,16 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
             for (int k = 0; k < 8; ++k) {
                 const bool mine = (eval_mask >> k) & 1u;
                 const unsigned m = __ballot_sync(kAll, mine);
-                if (mine) items.item[wv][total + __popc(m & lanes_below())] = (uint16_t)(k << 6 | (q0 + lane));
+                if (mine) items.item[wv & 1][total + __popc(m & lanes_below())] = (uint16_t)(k << 6 | (q0 + lane));
                 total += __popc(m);
             }
-            __syncwarp();
+            if constexpr (NW == kBlockY) {
+                __syncwarp();
+            } else { /* an owner's windows go to every second warp, view by view */
+                if (owner && lane == 0) items.count[wv] = total;
+                __syncthreads();
+                total = items.count[wv & 1];
+            }
         } else {
             const int r = round - 1;
             bool mine = false;
@@ -1192,16 +1205,16 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
             }
             eval_mask = mine ? 1u : 0u;
             const unsigned m = __ballot_sync(kAll, mine);
-            if (lane == 0) items.count[wv] = __popc(m);
+            if (owner && lane == 0) items.count[wv] = __popc(m);
             __syncthreads();
             if (mine) items.item[0][(wv ? items.count[0] : 0) + __popc(m & lanes_below())] = (uint16_t)(q0 + lane);
             total = items.count[0] + items.count[1];
             __syncthreads();
         }
-        const uint16_t *list = items.item[round == 0 ? wv : 0];
-        const int step = round == 0 ? 1 : kBlockY;
+        const uint16_t *list = items.item[round == 0 ? wv & 1 : 0];
+        const int step = round == 0 ? NW / kBlockY : NW;
 #pragma unroll 1
-        for (int v = round == 0 ? 0 : wv; v < S; v += step)
+        for (int v = round == 0 ? wv / kBlockY : wv; v < S; v += step)
 #pragma unroll 1
             for (int base = 0; base < total; base += 32) {
                 const bool need = base + lane < total;
@@ -1236,13 +1249,13 @@ __device__ __forceinline__ void prop_dirs_body(const PMArgs &a, int iter, const 
 
 /* WW: pixels of one colour per warp row (the half-step tile, tuned per view
  * size by the batched form; 8 elsewhere) */
-template <int WW>
-__global__ void __launch_bounds__(kBlock, HPM_P1_MIN_BLOCKS) k_prop_dirs(const __grid_constant__ PMArgs a, int iter,
-                                                                          int color)
+template <int WW, int NW>
+__global__ void __launch_bounds__(kBlockX *NW, NW == kBlockY ? HPM_P1_MIN_BLOCKS : kWideWarps / NW)
+    k_prop_dirs(const __grid_constant__ PMArgs a, int iter, int color)
 {
     __shared__ PatchMem<WW> sPatch;
     __shared__ DirItems sItems;
-    prop_dirs_body(a, iter, sPatch.load(a, color), sItems);
+    prop_dirs_body<WW, NW>(a, iter, sPatch.template load<NW>(a, color), sItems);
 }
 
 /* What the selection hands to the refinement, per pixel (rf_* in PMArgs):
@@ -1527,15 +1540,24 @@ __global__ void __launch_bounds__(kBlock, HPM_P3_MIN_BLOCKS) k_prop_select(const
     prop_select_body<SMAX, ACMM>(a, iter, px, py);
 }
 
-/* Shared memory of the refinement, per warp: its pixels' candidate planes and
- * the weighted sums of their costs; per block, the pixels whose winner's cost vector is
- * not complete yet. */
-template <int NC>
+/* Shared memory of the refinement, per owner warp: its pixels' candidate
+ * planes and the weighted sums of their costs; per block, the pixels whose
+ * winner's cost vector is not complete yet. */
+template <int NC, int NW>
 struct RefineItems {
     float4 cand[kBlockY][NC][32];
     float cost[kBlockY][NC][32];
-    uint8_t rank[kBlockY][kBlock];
+    uint8_t rank[NW][kBlock];
     uint32_t missing[kBlock];
+};
+
+/* With more warps than owners also the windows' statistics, the pixels that
+ * weigh each view, and (dynamic) each candidate's cost in each
+ * view, which the owners sum in the views' order. */
+struct RefineShare {
+    RefStats stats[kBlock];
+    uint8_t rank[kBlockY][kMaxSrc][32];
+    uint8_t count[kBlockY][kMaxSrc];
 };
 
 /* PROP: the prior-net form, whose network proposal a.proposals[center] is a
@@ -1545,25 +1567,29 @@ struct RefineItems {
  * ACMM: the ACMM+NESP variant (ACMM.cu:623-667): geometric weight 0.2 on the
  * refined hypotheses, and in a hierarchy pass the threshold rule on the
  * result.  A separate instantiation. */
-template <bool PROP, bool ACMM, int WW>
+template <bool PROP, bool ACMM, int WW, int NW>
 __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, const Patch<WW> &patch,
-                                                 RefineItems<PROP ? 6 : 5> &items)
+                                                 RefineItems<PROP ? 6 : 5, NW> &items, RefineShare *share,
+                                                 float *costs)
 {
     constexpr float kGeomW = ACMM ? 0.2f : 0.1f; /* HPM.cu:1189; ACMM.cu:651 */
     constexpr int NC = PROP ? 6 : 5;
     const int W = a.W, S = a.n - 1;
-    const int lane = threadIdx.x, wv = threadIdx.y, q0 = wv * kBlockX;
+    /* the first two warps own the block's pixels, others only score */
+    const int lane = threadIdx.x, wv = threadIdx.y & 1, q0 = wv * kBlockX;
+    const bool owner = NW == kBlockY || threadIdx.y < kBlockY;
     int px = patch.x(q0 + lane), py = patch.y(q0 + lane);
-    const bool act = px < W && py < a.rows_cov;
-    /* lanes outside the image stay for the block's windows, on a pixel
-     * inside, with no view weight and no write */
+    const bool act = owner && px < W && py < a.rows_cov;
+    /* lanes outside the image (and warps that own none) stay for the block's
+     * windows, on a pixel inside, with no view weight and no write */
     px = min(px, W - 1);
     py = min(py, a.H - 1);
     const int center = py * W + px;
     const Slot sl = slot_of(a, px, py);
     const HpmCamera &cam = a.cam[0];
     /* PlaneHypothesisRefinement, HPM.cu:1143-1220 */
-    const RefStats rs = ref_window(patch.win(q0 + lane));
+    RefStats rs = {0.0f, 0.0f, 0.0f};
+    if (owner) rs = ref_window(patch.win(q0 + lane));
     float4 plane = a.rf_plane[sl.hc];
     const float4 state = a.rf_state[sl.hc];
     float cost = state.x, depth_now = state.y, restricted_cost = state.z;
@@ -1625,58 +1651,98 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, cons
         for (int i = 0; i < 5; ++i) {
             float4 c = normals[i];
             c.w = distance_to_origin(cam, px, py, depths[i], c);
-            items.cand[wv][i][lane] = c;
+            if (owner) items.cand[wv][i][lane] = c;
             cand_depth[i] = depths[i];
         }
         if constexpr (PROP) {
             const float4 c = a.proposals[center];
-            items.cand[wv][5][lane] = c;
+            if (owner) items.cand[wv][5][lane] = c;
             cand_depth[5] = depth_from_plane(cam, c, px, py);
         }
-#pragma unroll
-        for (int i = 0; i < NC; ++i) items.cost[wv][i][lane] = 0.0f;
-#pragma unroll 1
-        for (int v = 0; v < S; ++v) {
-            /* the candidates of the pixels that weigh this view, packed: a
-             * pixel's together, candidates 0 and 2 (which share the random
-             * depth, hence the window centre) and 1, 3, 4 (at or near the
-             * current depth) next to each other, so that windows with the
-             * same centre meet in the texture cache */
-            const float weight = view_weight(vw_lo, vw_hi, v);
-            const bool selected = weight > 0.0f;
-            const unsigned m = __ballot_sync(kAll, selected);
-            if (m == 0) continue;
-            const int total = __popc(m) * NC;
-            if (selected) items.rank[wv][__popc(m & lanes_below())] = (uint8_t)lane;
-            __syncwarp();
-#pragma unroll 1
-            for (int base = 0; base < total; base += 32) {
-                const bool need = base + lane < total;
-                const int j = need ? base + lane : 0, n = j / NC, p = items.rank[wv][n], q = q0 + p;
-                const int i = (0x543120 >> (4 * (j - n * NC))) & 15;
-                const RefStats st = stats_of(rs, p);
-                const int hc = __shfl_sync(kAll, sl.hc, p);
-                const float w = __shfl_sync(kAll, weight, p);
-                const float4 h = items.cand[wv][i][p];
-                const int qx = patch.x(q), qy = patch.y(q);
-                /* the geometric term's source depth comes in under the window */
-                float spt[2], depth = 0.0f;
-                if (a.geom && need) {
-                    float P[3];
-                    geom_point(a, h, qx, qy, P);
-                    depth = geom_source(a, v + 1, P, spt);
-                }
-                float c = ncc_quad(a, v + 1, qx, qy, need, h, patch.win(q), st);
-                if (need) {
-                    __stcs(&a.cand_costs[(size_t)((kRefineRow + i) * S + v) * sl.nh + hc], c);
-                    if (a.geom) {
-                        c = __fmaf_rn(kGeomW, geom_distance(a, v + 1, qx, qy, spt, depth), c);
-                        count_geom(a, 1);
-                    }
-                    items.cost[wv][i][p] = __fmaf_rn(w, c, items.cost[wv][i][p]);
+        /* one window: its cost into the hand-off row; with the geometric term */
+        auto score = [&](int v, int i, int q, bool need, const RefStats &st) -> float {
+            const float4 h = items.cand[q >> 5][i][q & 31];
+            const int qx = patch.x(q), qy = patch.y(q);
+            /* the geometric term's source depth comes in under the window */
+            float spt[2], depth = 0.0f;
+            if (a.geom && need) {
+                float P[3];
+                geom_point(a, h, qx, qy, P);
+                depth = geom_source(a, v + 1, P, spt);
+            }
+            float c = ncc_quad(a, v + 1, qx, qy, need, h, patch.win(q), st);
+            if (need) {
+                __stcs(&a.cand_costs[(size_t)((kRefineRow + i) * S + v) * sl.nh + ((qy * W + qx) >> 1)], c);
+                if (a.geom) {
+                    c = __fmaf_rn(kGeomW, geom_distance(a, v + 1, qx, qy, spt, depth), c);
+                    count_geom(a, 1);
                 }
             }
-            __syncwarp();
+            return c;
+        };
+        /* the candidates of the pixels that weigh a view, packed: a pixel's
+         * together, candidates 0 and 2 (which share the random depth, hence
+         * the window centre) and 1, 3, 4 (at or near the current depth) next
+         * to each other, so that windows with the same centre meet in the
+         * texture cache */
+        if constexpr (NW == kBlockY) {
+#pragma unroll
+            for (int i = 0; i < NC; ++i) items.cost[wv][i][lane] = 0.0f;
+#pragma unroll 1
+            for (int v = 0; v < S; ++v) {
+                const float weight = view_weight(vw_lo, vw_hi, v);
+                const bool selected = weight > 0.0f;
+                const unsigned m = __ballot_sync(kAll, selected);
+                if (m == 0) continue;
+                const int total = __popc(m) * NC;
+                if (selected) items.rank[wv][__popc(m & lanes_below())] = (uint8_t)lane;
+                __syncwarp();
+#pragma unroll 1
+                for (int base = 0; base < total; base += 32) {
+                    const bool need = base + lane < total;
+                    const int j = need ? base + lane : 0, n = j / NC, p = items.rank[wv][n];
+                    const int i = (0x543120 >> (4 * (j - n * NC))) & 15;
+                    const RefStats st = stats_of(rs, p);
+                    const float w = __shfl_sync(kAll, weight, p);
+                    const float c = score(v, i, q0 + p, need, st);
+                    if (need) items.cost[wv][i][p] = __fmaf_rn(w, c, items.cost[wv][i][p]);
+                }
+                __syncwarp();
+            }
+        } else {
+            if (owner) {
+                share->stats[q0 + lane] = rs;
+                for (int v = 0; v < S; ++v) {
+                    const bool selected = (tsv >> v) & 1u;
+                    const unsigned m = __ballot_sync(kAll, selected);
+                    if (selected) share->rank[wv][v][__popc(m & lanes_below())] = (uint8_t)lane;
+                    if (lane == 0) share->count[wv][v] = (uint8_t)__popc(m);
+                }
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int v = threadIdx.y / kBlockY; v < S; v += NW / kBlockY) {
+                const int total = share->count[wv][v] * NC;
+#pragma unroll 1
+                for (int base = 0; base < total; base += 32) {
+                    const bool need = base + lane < total;
+                    const int j = need ? base + lane : 0, n = j / NC, q = q0 + share->rank[wv][v][n];
+                    const int i = (0x543120 >> (4 * (j - n * NC))) & 15;
+                    const float c = score(v, i, q, need, share->stats[q]);
+                    if (need) costs[(v * NC + i) * kBlock + q] = c;
+                }
+            }
+            __syncthreads();
+            if (owner) {
+#pragma unroll
+                for (int i = 0; i < NC; ++i) {
+                    float sum = 0.0f;
+                    for (int v = 0; v < S; ++v)
+                        if ((tsv >> v) & 1u)
+                            sum = __fmaf_rn(view_weight(vw_lo, vw_hi, v), costs[(v * NC + i) * kBlock + q0 + lane], sum);
+                    items.cost[wv][i][lane] = sum;
+                }
+            }
         }
         if (a.counters && tsv) atomicAdd(&a.counters[0], (unsigned long long)(NC * __popc(tsv)));
 #pragma unroll
@@ -1719,27 +1785,29 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, cons
     const bool took = act && best_row >= kRefineRow && best_row != kRowCurrent;
     const uint32_t all = S == 32 ? kAll : (1u << S) - 1u;
     __syncthreads();
-    items.cand[wv][0][lane] = plane;
-    items.cost[wv][0][lane] = rs.inv;
-    items.cost[wv][1][lane] = rs.mean;
-    items.cost[wv][2][lane] = rs.var;
-    items.missing[q0 + lane] = took ? all & ~tsv : 0u;
+    if (owner) {
+        items.cand[wv][0][lane] = plane;
+        items.cost[wv][0][lane] = rs.inv;
+        items.cost[wv][1][lane] = rs.mean;
+        items.cost[wv][2][lane] = rs.var;
+        items.missing[q0 + lane] = took ? all & ~tsv : 0u;
+    }
     __syncthreads();
 #pragma unroll 1
-    for (int v = wv; v < S; v += kBlockY) {
+    for (int v = threadIdx.y; v < S; v += NW) {
         int total = 0;
 #pragma unroll
         for (int half = 0; half < kBlockY; ++half) {
             const bool mine = (items.missing[half * kBlockX + lane] >> v) & 1u;
             const unsigned m = __ballot_sync(kAll, mine);
-            if (mine) items.rank[wv][total + __popc(m & lanes_below())] = (uint8_t)(half * kBlockX + lane);
+            if (mine) items.rank[threadIdx.y][total + __popc(m & lanes_below())] = (uint8_t)(half * kBlockX + lane);
             total += __popc(m);
         }
         __syncwarp();
 #pragma unroll 1
         for (int base = 0; base < total; base += 32) {
             const bool need = base + lane < total;
-            const int q = need ? items.rank[wv][base + lane] : 0, qw = q >> 5, p = q & 31;
+            const int q = need ? items.rank[threadIdx.y][base + lane] : 0, qw = q >> 5, p = q & 31;
             const RefStats st = {items.cost[qw][0][p], items.cost[qw][1][p], items.cost[qw][2][p]};
             const int qx = patch.x(q), qy = patch.y(q);
             const float c = ncc_quad(a, v + 1, qx, qy, need, items.cand[qw][0][p], patch.win(q), st);
@@ -1757,13 +1825,20 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, cons
         if (!took || ((tsv >> v) & 1u)) *cache_at(a, v, sl) = CAG(best_row, v);
 }
 
-template <bool PROP, int WW, bool ACMM>
-__global__ void __launch_bounds__(kBlock, HPM_P2_MIN_BLOCKS) k_prop_refine(const __grid_constant__ PMArgs a, int iter,
-                                                                            int color)
+template <bool PROP, int WW, bool ACMM, int NW>
+__global__ void __launch_bounds__(kBlockX *NW, NW == kBlockY ? HPM_P2_MIN_BLOCKS : kWideWarps / NW)
+    k_prop_refine(const __grid_constant__ PMArgs a, int iter, int color)
 {
     __shared__ PatchMem<WW> sPatch;
-    __shared__ RefineItems<PROP ? 6 : 5> sItems;
-    prop_refine_body<PROP, ACMM, WW>(a, iter, sPatch.load(a, color), sItems);
+    __shared__ RefineItems<PROP ? 6 : 5, NW> sItems;
+    const Patch<WW> patch = sPatch.template load<NW>(a, color);
+    if constexpr (NW == kBlockY) {
+        prop_refine_body<PROP, ACMM, WW, NW>(a, iter, patch, sItems, nullptr, nullptr);
+    } else {
+        __shared__ RefineShare sShare;
+        extern __shared__ float sCosts[]; /* [S][candidates][kBlock] */
+        prop_refine_body<PROP, ACMM, WW, NW>(a, iter, patch, sItems, &sShare, sCosts);
+    }
 }
 #undef CAG_PUT
 #undef CAG
@@ -1899,36 +1974,65 @@ __global__ void k_tap_samples(const __grid_constant__ PMArgs a, const float4 *pl
     }
 }
 
-template <int SMAX, int WW>
-cudaError_t launch_prop_t(const PMArgs &a, int iter, int color, cudaStream_t s)
+template <bool PROP, int WW, bool ACMM, int NW>
+cudaError_t launch_refine(const PMArgs &a, int iter, int color, dim3 grid, cudaStream_t s)
 {
-    constexpr int WH = 32 / WW;
-    const dim3 grid((a.W + 2 * WW - 1) / (2 * WW), (a.rows_cov + 2 * WH - 1) / (2 * WH)), b(kBlockX, kBlockY);
-    k_prop_dirs<WW><<<grid, b, 0, s>>>(a, iter, color);
+    size_t bytes = 0;
+    if constexpr (NW > kBlockY) {
+        bytes = sizeof(float) * (size_t)(a.n - 1) * (PROP ? 6 : 5) * kBlock;
+        const cudaError_t e = cudaFuncSetAttribute(k_prop_refine<PROP, WW, ACMM, NW>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+    }
+    k_prop_refine<PROP, WW, ACMM, NW><<<grid, dim3(kBlockX, NW), bytes, s>>>(a, iter, color);
+    return cudaGetLastError();
+}
+
+template <int SMAX, int WW, int NW>
+cudaError_t launch_prop_t(const PMArgs &a, int iter, int color, dim3 grid, cudaStream_t s)
+{
+    k_prop_dirs<WW, NW><<<grid, dim3(kBlockX, NW), 0, s>>>(a, iter, color);
+    const dim3 b(kBlockX, kBlockY);
     if constexpr (WW == 8) { /* the ACMM+NESP variant runs the default tile */
         if (a.acmm) {
             k_prop_select<SMAX, WW, true><<<grid, b, 0, s>>>(a, iter, color);
-            k_prop_refine<false, WW, true><<<grid, b, 0, s>>>(a, iter, color);
-            return cudaGetLastError();
+            return launch_refine<false, WW, true, NW>(a, iter, color, grid, s);
         }
     }
     k_prop_select<SMAX, WW, false><<<grid, b, 0, s>>>(a, iter, color);
-    if (a.proposals)
-        k_prop_refine<true, WW, false><<<grid, b, 0, s>>>(a, iter, color);
-    else
-        k_prop_refine<false, WW, false><<<grid, b, 0, s>>>(a, iter, color);
-    return cudaGetLastError();
+    return a.proposals ? launch_refine<true, WW, false, NW>(a, iter, color, grid, s)
+                       : launch_refine<false, WW, false, NW>(a, iter, color, grid, s);
+}
+
+/* Warps per block of 64 pixels.  Two where the grid fills the GPU; on small
+ * images, where a block's chain of windows is all there is to wait for, more
+ * warps share them: eight while two such blocks per SM hold the grid (148 SMs),
+ * four while four do.  A pass in ms with 2, 4 and 8 warps, by blocks: 54 0.80,
+ * 0.58, 0.51; 247 1.85, 1.43, 1.28; 294 1.86, 1.45, 1.30; 345 3.81, 2.96, 3.01;
+ * 486 1.29, 1.14, 1.35; 600 2.32, 2.28, 2.39; 950 2.94, 3.62, 4.58. */
+constexpr long long kBlocks8 = 2 * 148, kBlocks4 = 4 * 148;
+template <int SMAX, int WW>
+cudaError_t launch_prop_n(const PMArgs &a, int iter, int color, cudaStream_t s)
+{
+    constexpr int WH = 32 / WW;
+    const dim3 grid((a.W + 2 * WW - 1) / (2 * WW), (a.rows_cov + 2 * WH - 1) / (2 * WH));
+    if constexpr (WW == 8) {
+        const long long blocks = (long long)grid.x * grid.y;
+        if (blocks <= kBlocks8) return launch_prop_t<SMAX, WW, 8>(a, iter, color, grid, s);
+        if (blocks <= kBlocks4) return launch_prop_t<SMAX, WW, 4>(a, iter, color, grid, s);
+    }
+    return launch_prop_t<SMAX, WW, kBlockY>(a, iter, color, grid, s);
 }
 
 template <int WW>
 cudaError_t launch_prop_w(const PMArgs &a, int iter, int color, cudaStream_t s)
 {
     const int S = a.n - 1;
-    if (S <= 4) return launch_prop_t<4, WW>(a, iter, color, s);
-    if (S <= 8) return launch_prop_t<8, WW>(a, iter, color, s);
-    if (S <= 12) return launch_prop_t<12, WW>(a, iter, color, s);
-    if (S <= 16) return launch_prop_t<16, WW>(a, iter, color, s);
-    return launch_prop_t<kMaxSrc, WW>(a, iter, color, s);
+    if (S <= 4) return launch_prop_n<4, WW>(a, iter, color, s);
+    if (S <= 8) return launch_prop_n<8, WW>(a, iter, color, s);
+    if (S <= 12) return launch_prop_n<12, WW>(a, iter, color, s);
+    if (S <= 16) return launch_prop_n<16, WW>(a, iter, color, s);
+    return launch_prop_n<kMaxSrc, WW>(a, iter, color, s);
 }
 
 }  // namespace

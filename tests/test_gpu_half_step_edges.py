@@ -4,7 +4,8 @@ A block of the half-step kernels updates a patch of 16x8 pixels (one colour:
 two warps of 8x4 lanes) and its lanes score windows for one another, so the
 sizes here leave lanes, rows of lanes, whole warps and most of a block without
 a pixel, and the source counts lie on both sides of the widths the selection
-is compiled for and of the 16 view weights per word."""
+is compiled for and of the 16 view weights per word.  Grids of up to 296 blocks
+run eight warps per block, up to 592 (the last size) four."""
 import math
 
 import numpy as np
@@ -17,7 +18,8 @@ import synthetic as syn
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("w,h,sources", [(7, 5, 1), (16, 8, 2), (17, 9, 3), (15, 41, 9), (33, 17, 13), (47, 12, 17)])
+@pytest.mark.parametrize("w,h,sources", [(7, 5, 1), (16, 8, 2), (17, 9, 3), (15, 41, 9), (33, 17, 13), (47, 12, 17),
+                                         (272, 201, 5)])
 @pytest.mark.parametrize("half_steps", [0, 2])
 def test_half_steps_at_the_edges_of_the_tiles(w, h, sources, half_steps):
     sc = syn.make_scene(40 + w, w, h, sources + 1, n_planes=4, low_texture=0.0, arc_step_deg=min(8.0, 32.0 / sources))
