@@ -59,14 +59,13 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
     px = bx * (2 * ww) + 2 * (lane % ww) + ((py + color) & 1);
 }
 
-/* Blocks per SM that the window kernels are compiled for.  At 7 (14 warps,
- * 144 registers) nothing spills and the blocks' shared memory leaves 92 KB or
- * more to the texture cache; 10 and 6 blocks are slower (k_prop_dirs at
- * 1600x1200 with 10 sources: 3.41 and 3.77 against 3.42 ms, at 641x481 with 4:
- * 0.318 and 0.327 against 0.300; k_prop_refine 1.60 against 1.57 and 0.161
- * against 0.151). */
+/* Blocks per SM that the window kernels are compiled for: 14 to 16 warps, so
+ * that nothing spills and the blocks' shared memory leaves 92 KB or more to
+ * the texture cache (1600x1200, 5 sources, at 7, 8, 9 and 10 blocks:
+ * k_prop_dirs 1.70, 1.68, 1.71, 1.73 ms, k_prop_refine 0.95, 0.96, 2.14, 2.13;
+ * 641x481 with 4 sources behaves alike). */
 #ifndef HPM_P1_MIN_BLOCKS
-#define HPM_P1_MIN_BLOCKS 7
+#define HPM_P1_MIN_BLOCKS 8
 #endif
 #ifndef HPM_P2_MIN_BLOCKS
 #define HPM_P2_MIN_BLOCKS 7
@@ -543,15 +542,16 @@ __device__ __forceinline__ float pick(float a, float b, unsigned sel)
  * cache.  Products and sums are paired into two-wide instructions, since the
  * issue slots are the next bound, with the roundings spelled out.
  *
- * The view goes through a shuffle so that the compiler takes it as the same
- * in all lanes: otherwise each texture instruction becomes a loop over the
- * distinct texture handles of its lanes (k_prop_refine at 1600x1200, 10
- * sources: 3.70 against 1.80 ms). */
+ * The view goes through a warp reduction, whose result the hardware keeps once
+ * per warp, so that the compiler takes it as the same in all lanes: otherwise
+ * each texture instruction becomes a loop over the distinct texture handles of
+ * its lanes (k_prop_refine at 1600x1200, 10 sources: 3.70 against 1.80 ms; a
+ * shuffle does it too, but k_prop_dirs then takes 1.76 against 1.68 ms with 5). */
 template <typename Win>
 __device__ __forceinline__ float ncc_quad(const PMArgs &a, int v, int px, int py, bool need, float4 h, const Win &win,
                                           const RefStats &rs)
 {
-    v = __shfl_sync(kAll, v, 0);
+    v = (int)__reduce_max_sync(kAll, (unsigned)v);
     const HpmCamera &sc = a.cam[v];
     float H[9];
     homography(a.cam[0], sc, a.pairs[v], h, H);
