@@ -63,7 +63,11 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
  * that nothing spills and the blocks' shared memory leaves 92 KB or more to
  * the texture cache (1600x1200, 5 sources, at 7, 8, 9 and 10 blocks:
  * k_prop_dirs 1.70, 1.68, 1.71, 1.73 ms, k_prop_refine 0.95, 0.96, 2.14, 2.13;
- * 641x481 with 4 sources behaves alike). */
+ * 641x481 with 4 sources behaves alike; k_init with 10 sources at 6, 8 and 10
+ * blocks: 1.05, 1.02, 1.67 ms). */
+#ifndef HPM_P0_MIN_BLOCKS
+#define HPM_P0_MIN_BLOCKS 8
+#endif
 #ifndef HPM_P1_MIN_BLOCKS
 #define HPM_P1_MIN_BLOCKS 8
 #endif
@@ -217,17 +221,40 @@ __device__ __forceinline__ float tap_weight(float spatial, float ref, float cent
 /* The reference window of a pixel: its weights in shared memory, written once
  * by ref_window ([row pair][column][thread]: the weights of two rows side by
  * side for the packed sums of ncc_quad), and its pixels, read at each use from
- * global memory (WinImage) or from a tile of the block's surroundings in
- * shared memory (WinTile).  Computing the weights again at each use would
- * halve the block's shared memory but costs more than the texture cache gains
- * (refinement at 1600x1200, 10 sources: 1.80 against 1.57 ms). */
-struct WinImage {
+ * a tile of the block's surroundings in shared memory (WinRow for blocks of
+ * whole rows, WinTile for half-steps).  Computing the weights again at each
+ * use would halve the block's shared memory but costs more than the texture
+ * cache gains (refinement at 1600x1200, 10 sources: 1.80 against 1.57 ms). */
+struct WinRow {
+    static constexpr int kRows = kBlockY + 10, kPitch = kBlockX + 10;
     const Spatial *sp;
-    float range_scale, mid;
-    float2 *w; /* this thread's column */
-    const float *img;
-    int W, H, px, py;
-    __device__ __forceinline__ float ref(int ti, int tj) const { return texel(img, W, H, px + 2 * ti - 5, py + 2 * tj - 5); }
+    float range_scale, mid; /* the pixel's own value */
+    float2 *w;              /* its column of weights */
+    const float *tile;      /* its first tap */
+    __device__ __forceinline__ float ref(int ti, int tj) const { return tile[2 * tj * kPitch + 2 * ti]; }
+};
+
+/* Shared memory of a 32 x 2 block's reference windows.  The tile is read once
+ * where 36 clamped loads a window came from global memory before, each with
+ * its own clamping (k_init at 1600x1200, 10 sources: 1.11 -> 1.02 ms, in
+ * geometric passes 0.96 -> 0.83; 641x481 with 4: 0.085 -> 0.074). */
+struct RowMem {
+    float2 w[kTaps / 2 * kBlock];
+    float tile[WinRow::kRows * WinRow::kPitch];
+    Spatial sp;
+
+    /* fills the tile (all threads; edges repeated) and the spatial terms;
+     * returns the window of the thread's pixel */
+    __device__ __forceinline__ WinRow load(const ViewDev &rv, float sigma_spatial, float sigma_color)
+    {
+        const int x0 = (int)blockIdx.x * kBlockX - 5, y0 = (int)blockIdx.y * kBlockY - 5;
+        const int tid = threadIdx.y * kBlockX + threadIdx.x;
+        for (int i = tid; i < WinRow::kRows * WinRow::kPitch; i += kBlock)
+            tile[i] = texel(rv.img, rv.w, rv.h, x0 + i % WinRow::kPitch, y0 + i / WinRow::kPitch);
+        spatial_terms(sigma_spatial, &sp);
+        const float *first = tile + threadIdx.y * WinRow::kPitch + threadIdx.x;
+        return {&sp, rcp_approx(2.0f * sigma_color * sigma_color), first[5 * WinRow::kPitch + 5], w + tid, first};
+    }
 };
 
 /* Half-step blocks: every tap of a pixel has the pixel's own checkerboard
@@ -447,12 +474,6 @@ __device__ __forceinline__ float2 warp(const float *H, float px, float py)
 /* ------------------------------------------------------------------ */
 /* Hoisted reference window                                            */
 /* ------------------------------------------------------------------ */
-
-__device__ __forceinline__ WinImage image_window(const PMArgs &a, const Spatial *sp, float2 *w, int px, int py)
-{
-    return {sp, rcp_approx(2.0f * a.sigma_color * a.sigma_color), texel(a.view[0].img, a.W, a.H, px, py), w,
-            a.view[0].img, a.W, a.H, px, py};
-}
 
 struct RefStats {
     float inv;  /* 1 / sum of weights */
@@ -809,14 +830,13 @@ __device__ __forceinline__ float *cache_at(const PMArgs &a, int v, const Slot &s
 }
 
 /* RandomInitialization, HPM.cu:510-558.  One thread per pixel. */
-__device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, const Spatial &sp, float2 *sW, float *sCV, int tid)
+__device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, const WinRow &win, float *sCV, int tid)
 {
     const bool act = px < a.W && py < a.H;
     /* lanes outside the image stay for the warp's windows, on a pixel inside */
     const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
     const int center = cy * a.W + cx;
     const HpmCamera &cam = a.cam[0];
-    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
     const RefStats rs = ref_window(win);
     Rng rng;
     rng.init(a.seed_lo, a.seed_hi, (uint32_t)center, 0u, a.salt);
@@ -877,14 +897,13 @@ __device__ __forceinline__ void init_body(const PMArgs &a, int px, int py, const
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_init(const __grid_constant__ PMArgs a)
+__global__ void __launch_bounds__(kBlock, HPM_P0_MIN_BLOCKS) k_init(const __grid_constant__ PMArgs a)
 {
-    __shared__ float2 sW[kTaps / 2 * kBlock];
+    __shared__ RowMem sRow;
     __shared__ float sCV[kMaxSrc * kBlock];
-    __shared__ Spatial sp;
-    spatial_terms(a.sigma_spatial, &sp);
     const int tid = threadIdx.y * kBlockX + threadIdx.x;
-    init_body(a, blockIdx.x * kBlockX + threadIdx.x, blockIdx.y * kBlockY + threadIdx.y, sp, sW, sCV, tid);
+    init_body(a, blockIdx.x * kBlockX + threadIdx.x, blockIdx.y * kBlockY + threadIdx.y,
+              sRow.load(a.view[0], a.sigma_spatial, a.sigma_color), sCV, tid);
 }
 
 /* Validity of the first site of direction k at extension round r (HPM.cu:1252-1445 and the
@@ -1948,15 +1967,12 @@ __global__ void k_filter(const __grid_constant__ PMArgs a, float4 *pl, const flo
 __global__ void __launch_bounds__(kBlock) k_cost_vectors(const __grid_constant__ PMArgs a, const float4 *planes,
                                                           float *out)
 {
-    __shared__ float2 sW[kTaps / 2 * kBlock];
-    __shared__ Spatial sp;
-    spatial_terms(a.sigma_spatial, &sp);
-    const int tid = threadIdx.y * kBlockX + threadIdx.x;
+    __shared__ RowMem sRow;
+    const WinRow win = sRow.load(a.view[0], a.sigma_spatial, a.sigma_color);
     const int px = blockIdx.x * kBlockX + threadIdx.x;
     const int py = blockIdx.y * kBlockY + threadIdx.y;
     const bool act = px < a.W && py < a.H;
     const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
-    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
     const RefStats rs = ref_window(win);
     const int c = cy * a.W + cx;
     const int S = a.n - 1;
@@ -1966,16 +1982,14 @@ __global__ void __launch_bounds__(kBlock) k_cost_vectors(const __grid_constant__
 __global__ void __launch_bounds__(kBlock) k_initial_costs(const __grid_constant__ PMArgs a, const float4 *planes,
                                                           float *cost, uint32_t *views)
 {
-    __shared__ float2 sW[kTaps / 2 * kBlock];
-    __shared__ Spatial sp;
-    spatial_terms(a.sigma_spatial, &sp);
+    __shared__ RowMem sRow;
+    const WinRow win = sRow.load(a.view[0], a.sigma_spatial, a.sigma_color);
     __shared__ float sCV[kMaxSrc * kBlock];
     const int tid = threadIdx.y * kBlockX + threadIdx.x;
     const int px = blockIdx.x * kBlockX + threadIdx.x;
     const int py = blockIdx.y * kBlockY + threadIdx.y;
     const bool act = px < a.W && py < a.H;
     const int cx = min(px, a.W - 1), cy = min(py, a.H - 1);
-    const WinImage win = image_window(a, &sp, sW + tid, cx, cy);
     const RefStats rs = ref_window(win);
     const int c = cy * a.W + cx;
     cost_vector(a, px, py, act, planes[c], win, rs, sCV + tid, kBlock);
