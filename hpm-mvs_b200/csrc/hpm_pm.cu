@@ -2044,9 +2044,13 @@ cudaError_t launch_refine(const PMArgs &a, int iter, int color, dim3 grid, cudaS
 {
     size_t bytes = 0;
     if constexpr (NW > kBlockY) {
-        bytes = sizeof(float) * (size_t)(a.n - 1) * (PROP ? 6 : 5) * kBlock;
+        constexpr size_t per_source = sizeof(float) * (PROP ? 6 : 5) * kBlock;
+        bytes = per_source * (a.n - 1);
+        /* the limit belongs to the kernel, not to the launch: the same value
+         * for every size, since another thread may launch with more sources */
         const cudaError_t e = cudaFuncSetAttribute(k_prop_refine<PROP, WW, ACMM, NW>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)(per_source * kMaxSrc));
         if (e != cudaSuccess) return e;
     }
     k_prop_refine<PROP, WW, ACMM, NW><<<grid, dim3(kBlockX, NW), bytes, s>>>(a, iter, color);

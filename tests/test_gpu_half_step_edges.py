@@ -7,6 +7,7 @@ a pixel, and the source counts lie on both sides of the widths the selection
 is compiled for and of the 16 view weights per word.  Grids of up to 296 blocks
 run eight warps per block, up to 592 (the last size) four."""
 import math
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -41,3 +42,28 @@ def test_half_steps_at_the_edges_of_the_tiles(w, h, sources, half_steps):
     close = np.isclose(gc[same], oc[same], rtol=1e-3, atol=1e-3, equal_nan=True)
     assert same.mean() >= least(0.999 if half_steps == 0 else 0.95), same.mean()
     assert close.mean() >= least(0.99), close.mean()
+
+
+def test_two_threads_with_different_source_counts():
+    """The refinement's shared memory follows the source count; contexts of two threads launch it side by side."""
+    def problem(sources):
+        sc = syn.make_scene(70, 48, 36, sources + 1, n_planes=4, low_texture=0.0, arc_step_deg=2.0)
+        imgs, cams = syn.view_set(sc, 0)
+        return imgs, cams, hb.default_params(sc.depth_min * 0.6, sc.depth_max * 1.2, seed=3)
+
+    def passes(inputs):
+        imgs, cams, p = inputs
+        maps = []
+        with hb.Context() as ctx:
+            ctx.set_views(imgs, cams)
+            for _ in range(60):  # each with its own random streams
+                ctx.run_partial(p, 2, False)
+                maps.append(ctx.get_result()[0])
+        return maps
+
+    inputs = [problem(2), problem(14)]
+    alone = [passes(k) for k in inputs]
+    with ThreadPoolExecutor(2) as pool:
+        got = list(pool.map(passes, inputs))
+    for one, other in zip(alone, got):
+        assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(one, other))
