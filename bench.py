@@ -61,10 +61,10 @@ BATCHED = dict(width=1920, height=1080, n_views=24, n_planes=20, n_spheres=5, lo
                sizes=[(1920, 1080)] * 8 + [(1600, 1200)] * 8 + [(960, 540)] * 8,
                name="batched scene")
 
-# DRAM traffic of one half-step (k_prop_dirs + k_prop_refine: read + write),
-# from an ncu capture of `bench.py --pass-case` (1600x1200, 10 sources), per
-# pixel: the hand-off buffers grow with the pixel count
-TRAFFIC_BYTES_PER_PX_HALF_STEP = (154.02 + 323.62 + 797.47 + 388.49) * 1e6 / (1600 * 1200)
+# DRAM traffic of one half-step (k_prop_dirs, k_prop_select, k_prop_refine: read +
+# write), from an ncu capture of a plain pass (1600x1200, 10 sources), per pixel:
+# the hand-off buffers grow with the pixel count
+TRAFFIC_BYTES_PER_PX_HALF_STEP = (163.31 + 297.12 + 548.03 + 126.86 + 527.53 + 226.96) * 1e6 / (1600 * 1200)
 GEOM_TERM_FLOPS = 120  # two projections (world point + camera, 3x3 each) and the reprojection distance
 TAPS, NCC_FLOPS_PER_TAP, FLOPS_PER_HYP_VIEW = 36, 34, 80
 
@@ -517,10 +517,10 @@ def run_ours(args, dist):
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
                      "traffic": TRAFFIC_BYTES_PER_PX_HALF_STEP * npx,
-                     "traffic_note": "DRAM bytes per half-step (k_prop_dirs + k_prop_refine) from the ncu capture "
-                                     "of bench.py --pass-case at 1600x1200 (10 sources), per pixel of the "
+                     "traffic_note": "DRAM bytes per half-step (k_prop_dirs + k_prop_select + k_prop_refine) from the "
+                                     "ncu capture of a plain pass at 1600x1200 (10 sources), per pixel of the "
                                      "workload",
-                     "kernel": "k_prop_dirs + k_prop_refine (one red/black half-step), timed with CUDA events "
+                     "kernel": "k_prop_dirs + k_prop_select + k_prop_refine (one red/black half-step), timed with CUDA events "
                                "in the plain form's timed steps",
                      "peak_source": "measured FP32 FMA probe (hpm_fp32_peak) of measured; "
                                     "MEASURED_PEAKS.json has no FP32 figure",
