@@ -413,7 +413,8 @@ int hpm_net_targets(int device, const HpmCamera *ref_cam, const float *depth, co
 
 /* Training loss of the head on n pixels (device buffers): masked relative
  * depth error plus lambda (1 - cos) of the normal; dy gets the output
- * gradient (BF16, 16 channels) times inv_count, *loss the loss sum. */
+ * gradient (BF16, 16 channels) times inv_count; the loss sum, taken in 64 bits
+ * and a fixed order, is added to *loss. */
 int hpm_net_loss(const float *out16, const float *t_depth, const float *t_normal, const uint8_t *t_mask, int n,
                  float dmin, float dmax, float lambda, float inv_count, void *dy, float *loss, void *stream);
 
