@@ -1783,8 +1783,9 @@ __device__ __forceinline__ void prop_refine_body(const PMArgs &a, int iter, cons
             }
         }
         if (a.counters && tsv) atomicAdd(&a.counters[0], (unsigned long long)(NC * __popc(tsv)));
+        /* by the owners alone: they write their sums without another barrier */
 #pragma unroll
-        for (int i = 0; i < NC; ++i) {
+        for (int i = 0; owner && i < NC; ++i) {
             const float tci = items.cost[wv][i][lane] / wn;
             const float4 ci = items.cand[wv][i][lane];
             const float depth_before = depth_from_plane(cam, ci, px, py);
