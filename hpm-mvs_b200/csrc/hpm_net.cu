@@ -167,10 +167,17 @@ __global__ void __launch_bounds__(128)
                         v[n / 2] = __floats2bfloat162_rn(fmaxf(__uint_as_float(r[n]) + bias[n], 0.0f),
                                                          fmaxf(__uint_as_float(r[n + 1]) + bias[n + 1], 0.0f));
                 } else {
+                    /* 16 bytes at a time where aux starts on 16 bytes, which
+                     * is not asked of it: a caller's view may start anywhere */
                     __align__(16) __nv_bfloat16 ax[COUT];
+                    if ((reinterpret_cast<uintptr_t>(aux) & 15u) == 0) {
 #pragma unroll
-                    for (int q = 0; q < COUT / 8; ++q)
-                        reinterpret_cast<uint4 *>(ax)[q] = reinterpret_cast<const uint4 *>(aux + o)[q];
+                        for (int q = 0; q < COUT / 8; ++q)
+                            reinterpret_cast<uint4 *>(ax)[q] = reinterpret_cast<const uint4 *>(aux + o)[q];
+                    } else {
+#pragma unroll
+                        for (int n = 0; n < COUT; ++n) ax[n] = aux[o + n];
+                    }
 #pragma unroll
                     for (int n = 0; n < COUT; n += 2) {
                         const float g0 = __bfloat162float(ax[n]) > 0.0f ? __uint_as_float(r[n]) : 0.0f;
