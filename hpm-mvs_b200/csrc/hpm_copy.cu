@@ -3,15 +3,24 @@
  *
  * A cudaMemcpyAsync of pageable memory goes through the driver's staging on
  * the calling thread: 11 GB/s in, and 5 GB/s out into pages that have not been
- * touched yet, with the GPU idle meanwhile.  Here a few threads copy 1 MB
- * chunks through their own pinned buffers (two each, so that a thread's copy
- * runs under its transfer); first touches of the destination are spread over
- * them as well.  11 images of 3200x2133 (300 MB) in: 27.0 -> 8.0 ms; planes
- * and costs of that size (137 MB) out: 23.5 -> 5.5 ms.  Small copies take the
- * plain way, where the threads cost more than they save (13 MB in: 1.3 against
- * 1.2 ms; 27 MB out into touched pages: 1.7 against 1.3 ms; 34 MB in: 1.8
- * against 3.1; 38 MB out: 1.5 against 1.9), and so does pinned or device
- * memory, which needs no staging.
+ * touched yet, with the GPU idle meanwhile (the driver lets one thread at a
+ * time through it, so more threads in it change nothing).  Here a few threads
+ * copy 1 MB chunks (smaller ones: 300 MB in 8.4 ms, with 512 KB 11.2, with
+ * 256 KB 14.9) through their own pinned buffers (two each, so that a thread's
+ * copy runs under its transfer); first touches of the destination are spread
+ * over them as well.  11 images of 3200x2133 (300 MB) in: 27.0 -> 8.0 ms;
+ * planes and costs of that size (137 MB) out: 23.5 -> 5.5 ms.  Small copies
+ * take the plain way, where the threads cost more than they save (13 MB in:
+ * 1.3 against 1.2 ms; 27 MB out into touched pages: 1.7 against 1.3 ms; 34 MB
+ * in: 1.8 against 3.1; 38 MB out: 1.5 against 1.9), and so does pinned or
+ * device memory, which needs no staging.
+ *
+ * The pinned buffers themselves take 11 to 25 ms to make, more than a copy of
+ * a few tens of MB saves, so a context that lives for one problem goes without
+ * them (worth_it).  A new context's first hpm_set_views in ms, with buffers
+ * made on the first large copy and now: 20 MB 19.2, 7.0; 38 MB 22.0, 9.0;
+ * 40 MB in 21 images 32.0, 18.9; 100 MB 28.4, 18.3; 300 MB 32.1, 32.9 (all
+ * plain: 38.0).
  */
 #include <string.h>
 
@@ -30,6 +39,7 @@ namespace {
 constexpr size_t kChunk = 1 << 20;
 constexpr int kMaxThreads = 8, kSlots = 2;
 constexpr size_t kMinIn = 16 << 20, kMinOut = 32 << 20;
+constexpr size_t kNowIn = 256 << 20, kNowOut = 128 << 20, kSoFar = 512 << 20;
 }  // namespace
 
 struct HostCopier {
@@ -70,6 +80,18 @@ HostCopier *copier_of(hpm_ctx *c)
     return h;
 }
 
+/* Whether a copy of `bytes` pageable bytes, large enough for the threads, gets
+ * pinned buffers to go through where the context has none yet: when this copy
+ * alone saves more than they cost, or when the copies that this context has
+ * made without them add up to a long-lived one's (bytes out count twice, as
+ * they save twice as much). */
+bool worth_it(hpm_ctx *c, size_t bytes, bool out)
+{
+    if (c->copier) return true;
+    c->staged_so_far += out ? 2 * bytes : bytes;
+    return bytes >= (out ? kNowOut : kNowIn) || c->staged_so_far >= kSoFar;
+}
+
 bool pageable(const void *p)
 {
     cudaPointerAttributes at;
@@ -106,7 +128,7 @@ cudaError_t copy(hpm_ctx *c, const CopyItem *items, int n, bool out)
             stage[i] = pageable(out ? items[i].dst : items[i].src);
             if (stage[i]) staged += items[i].bytes;
         }
-        if (staged >= least && !copier_of(c)) staged = 0;
+        if (staged >= least && (!worth_it(c, staged, out) || !copier_of(c))) staged = 0;
         if (staged >= least)
             for (int i = 0; i < n; ++i)
                 for (size_t at = 0; stage[i] && at < items[i].bytes; at += kChunk)

@@ -17,7 +17,7 @@ struct CopyItem {
     size_t bytes;
 };
 
-struct HostCopier; /* a context's pinned buffers, made on the first large copy */
+struct HostCopier; /* a context's pinned buffers, made when its copies are worth them */
 void host_copier_free(HostCopier *h);
 
 /* Queues the items on the context's stream; sources may be host (pageable or
