@@ -18,7 +18,7 @@ __global__ void k_jbu(const float *__restrict__ guide, int cols, int rows, const
 {
     const JbuTaps taps = jbu_block_taps(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
-    const int py = blockIdx.y * blockDim.y + threadIdx.y;
+    const int py = jbu_block_row() + threadIdx.y;
     if (px >= cols || py >= rows) return;
     float4 n = jbu_pixel(guide, cols, rows, coarse, s_cols, s_rows, image_scale, px, py, taps);
     const size_t c = (size_t)py * cols + px;
@@ -33,8 +33,8 @@ cudaError_t launch_jbu(const float *guide, int cols, int rows, const float *coar
                        int s_cols, int s_rows, int image_scale, float *out_depth, float4 *out_normal, cudaStream_t s)
 {
     (void)coarse_depth; /* packed into coarse_normal.w by the caller */
-    dim3 b(kJbuBlockX, kJbuBlockY), g((cols + kJbuBlockX - 1) / kJbuBlockX, (rows + kJbuBlockY - 1) / kJbuBlockY);
-    k_jbu<<<g, b, 0, s>>>(guide, cols, rows, coarse_normal, s_cols, s_rows, image_scale, out_depth, out_normal);
+    k_jbu<<<jbu_grid(cols, rows), dim3(kJbuBlockX, kJbuBlockY), 0, s>>>(guide, cols, rows, coarse_normal, s_cols, s_rows,
+                                                                        image_scale, out_depth, out_normal);
     return cudaGetLastError();
 }
 

@@ -36,6 +36,15 @@ namespace hpm {
 constexpr int kJbuBlockX = 32, kJbuBlockY = 8;
 constexpr float kJbuReach2 = 45.0f; /* expf(-2 * 45) is 0 in FP32 */
 
+/* A grid's y ends at 65,535, so the block rows beyond continue along z (524,280
+ * rows and more of a narrow image). */
+inline dim3 jbu_grid(int cols, int rows)
+{
+    const unsigned n = ((unsigned)rows + kJbuBlockY - 1) / kJbuBlockY;
+    return dim3(((unsigned)cols + kJbuBlockX - 1) / kJbuBlockX, n < 65535u ? n : 65535u, (n + 65534u) / 65535u);
+}
+__device__ __forceinline__ int jbu_block_row() { return (blockIdx.z * gridDim.y + blockIdx.y) * kJbuBlockY; }
+
 enum JbuTaps { kJbuAll, kJbuNear, kJbuInner };
 
 __device__ __forceinline__ int jbu_coarse(float v, int n)
@@ -52,7 +61,7 @@ __device__ __forceinline__ JbuTaps jbu_block_taps(const float *__restrict__ guid
 {
     const float scale = (float)(1.0 * s_cols / cols);
     const int nn = (image_scale * image_scale + 1) / 2;
-    const int x0 = blockIdx.x * kJbuBlockX, y0 = blockIdx.y * kJbuBlockY;
+    const int x0 = blockIdx.x * kJbuBlockX, y0 = jbu_block_row();
     const int x1 = min(x0 + kJbuBlockX, cols) - 1, y1 = min(y0 + kJbuBlockY, rows) - 1;
     const int tid = threadIdx.y * kJbuBlockX + threadIdx.x;
     bool finite = true;

@@ -51,7 +51,7 @@ __global__ void k_jbu_noalloc(const float *__restrict__ guide, int cols, int row
 {
     const hpm::JbuTaps taps = hpm::jbu_block_taps(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
-    const int py = blockIdx.y * blockDim.y + threadIdx.y;
+    const int py = hpm::jbu_block_row() + threadIdx.y;
     if (px >= cols || py >= rows) return;
     const float4 n = hpm::jbu_pixel(guide, cols, rows, coarse, s_cols, s_rows, image_scale, px, py, taps);
     const size_t o = (size_t)py * cols + px;
@@ -114,11 +114,10 @@ extern "C" int hpm_jbu_noalloc(int device, const float *guide, int cols, int row
         const float4 *coarse = scratch;
         int image_scale_arg = image_scale;
         const dim3 block(hpm::kJbuBlockX, hpm::kJbuBlockY);
-        const dim3 grid((cols + block.x - 1) / block.x, (rows + block.y - 1) / block.y);
         void *args[] = {(void *)&guide,  (void *)&cols,   (void *)&rows,           (void *)&coarse,
                         (void *)&s_cols, (void *)&s_rows, (void *)&image_scale_arg, (void *)&out_depth,
                         (void *)&out_normal};
-        if (cudaLaunchKernel((const void *)k_jbu_noalloc, grid, block, args, 0, s) != cudaSuccess)
+        if (cudaLaunchKernel((const void *)k_jbu_noalloc, hpm::jbu_grid(cols, rows), block, args, 0, s) != cudaSuccess)
             return HPM_ERR_CUDA;
     }
     return HPM_OK;
