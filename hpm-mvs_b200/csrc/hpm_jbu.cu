@@ -12,11 +12,12 @@
 namespace hpm {
 namespace {
 
+template <bool CUT>
 __global__ void k_jbu(const float *__restrict__ guide, int cols, int rows, const float4 *__restrict__ coarse,
                       int s_cols, int s_rows, int image_scale, float *__restrict__ out_depth,
                       float4 *__restrict__ out_normal)
 {
-    const JbuTaps taps = jbu_block_taps(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
+    const JbuTaps taps = jbu_block_taps<CUT>(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
     const int py = jbu_block_row() + threadIdx.y;
     if (px >= cols || py >= rows) return;
@@ -33,8 +34,9 @@ cudaError_t launch_jbu(const float *guide, int cols, int rows, const float *coar
                        int s_cols, int s_rows, int image_scale, float *out_depth, float4 *out_normal, cudaStream_t s)
 {
     (void)coarse_depth; /* packed into coarse_normal.w by the caller */
-    k_jbu<<<jbu_grid(cols, rows), dim3(kJbuBlockX, kJbuBlockY), 0, s>>>(guide, cols, rows, coarse_normal, s_cols, s_rows,
-                                                                        image_scale, out_depth, out_normal);
+    auto *kernel = jbu_cuts(image_scale) ? k_jbu<true> : k_jbu<false>;
+    kernel<<<jbu_grid(cols, rows), dim3(kJbuBlockX, kJbuBlockY), 0, s>>>(guide, cols, rows, coarse_normal, s_cols, s_rows,
+                                                                         image_scale, out_depth, out_normal);
     return cudaGetLastError();
 }
 

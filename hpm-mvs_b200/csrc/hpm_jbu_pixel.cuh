@@ -18,13 +18,15 @@
  *
  * What bounds it is the arithmetic of the (s*s+1)^2 taps (two expf each).  A
  * tap whose coarse sample is more than sqrt(45) coarse pixels away has a
- * spatial weight exp(-90) or less, which is zero in FP32, and adding zero
- * changes no sum: at scale 4 these are 152 of the 289 taps.  They are left
- * out where every value in reach of the block is finite (a weight of zero
- * times an infinity is not zero); elsewhere all taps are taken.  Away from
+ * spatial weight exp(-90) or less, which the build's flush of subnormals makes
+ * zero, and adding zero changes no sum: at scale 4 these are 152 of the 289
+ * taps.  They are left out where every value in reach of the block is finite
+ * (a weight of zero times an infinity is not zero); elsewhere all taps are
+ * taken, and at scales below 4, whose windows hold few such taps or none, so
+ * that looking for them costs more than it saves (jbu_cuts).  Away from
  * the borders, with a power of two as the scale, coordinates are exact and a
  * row's taps are a plain run of the coarse grid, without conversions and
- * clamps.  1600x1200 from 400x300: 775 us with all taps, 430 us now, the
+ * clamps.  1600x1200 from 400x300: 760 us with all taps, 423 us now, the
  * same bits.
  */
 #pragma once
@@ -34,7 +36,6 @@
 namespace hpm {
 
 constexpr int kJbuBlockX = 32, kJbuBlockY = 8;
-constexpr float kJbuReach2 = 45.0f; /* expf(-2 * 45) is 0 in FP32 */
 
 /* A grid's y ends at 65,535, so the block rows beyond continue along z (524,280
  * rows and more of a narrow image). */
@@ -45,6 +46,12 @@ inline dim3 jbu_grid(int cols, int rows)
 }
 __device__ __forceinline__ int jbu_block_row() { return (blockIdx.z * gridDim.y + blockIdx.y) * kJbuBlockY; }
 
+/* Squared distance in coarse pixels beyond which a spatial weight is zero:
+ * exp(-90) is where subnormals are flushed (the Makefile's --use_fast_math), and
+ * exp(-104) rounds to zero in any FP32.  Asked of expf itself, so that the
+ * header is right under either build. */
+__device__ __forceinline__ float jbu_reach2() { return expf(-90.0f) == 0.0f ? 45.0f : 52.0f; }
+
 enum JbuTaps { kJbuAll, kJbuNear, kJbuInner };
 
 __device__ __forceinline__ int jbu_coarse(float v, int n)
@@ -53,12 +60,21 @@ __device__ __forceinline__ int jbu_coarse(float v, int n)
     return r > 0 ? (r < n ? r : n - 1) : 0;
 }
 
+/* The scales whose kernel looks for the taps out of reach (CUT).  1600x1200
+ * with all taps and with those in reach, by scale: 2 85 and 91 us (no tap is
+ * out of reach), 3 316 and 386, 4 760 and 423 (775 and 615 for 1601x1201, whose
+ * coordinates are not exact), 5 1829 and 779.  A kernel of its own for the rest:
+ * as a branch of one kernel, all taps at scale 3 took 351 us. */
+inline bool jbu_cuts(int image_scale) { return image_scale >= 4; }
+
 /* How the block's pixels take their taps (the same answer in all threads; all
  * must call). */
+template <bool CUT>
 __device__ __forceinline__ JbuTaps jbu_block_taps(const float *__restrict__ guide, int cols, int rows,
                                                   const float4 *__restrict__ coarse, int s_cols, int s_rows,
                                                   int image_scale)
 {
+    if constexpr (!CUT) return kJbuAll;
     const float scale = (float)(1.0 * s_cols / cols);
     const int nn = (image_scale * image_scale + 1) / 2;
     const int x0 = blockIdx.x * kJbuBlockX, y0 = jbu_block_row();
@@ -101,6 +117,30 @@ struct JbuSums {
     }
 };
 
+/* The window's taps with clamped coordinates: all, or those in reach. */
+template <bool NEAR>
+__device__ __forceinline__ void jbu_window(const float *__restrict__ guide, int cols, int rows,
+                                           const float4 *__restrict__ coarse, int s_cols, int s_rows, int nn, int px,
+                                           int py, float ox, float oy, float ref_pix, JbuSums &s)
+{
+    const float reach2 = jbu_reach2();
+    for (int j = -nn; j <= nn; ++j) {
+        const int ry = jbu_coarse(oy + (float)j, s_rows);
+        const int rys = min(max(py + j, 0), rows - 1);
+        const float dy = oy - (float)ry;
+        if (NEAR && dy * dy > reach2) continue;
+        const float *grow = guide + (size_t)rys * cols;
+        for (int i = -nn; i <= nn; ++i) {
+            const int rx = jbu_coarse(ox + (float)i, s_cols);
+            const float dx = ox - (float)rx;
+            const float dis = dx * dx + dy * dy;
+            if (NEAR && dis > reach2) continue;
+            const int rxs = min(max(px + i, 0), cols - 1);
+            s.add(__ldg(coarse + (size_t)ry * s_cols + rx), dis, ref_pix, __ldg(grow + rxs));
+        }
+    }
+}
+
 /* Returns (nx, ny, nz, depth) of fine pixel (px, py). */
 __device__ __forceinline__ float4 jbu_pixel(const float *__restrict__ guide, int cols, int rows,
                                             const float4 *__restrict__ coarse, int s_cols, int s_rows,
@@ -112,13 +152,14 @@ __device__ __forceinline__ float4 jbu_pixel(const float *__restrict__ guide, int
     const float ref_pix = __ldg(guide + (size_t)py * cols + px);
     JbuSums s = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     if (taps == kJbuInner) {
+        const float reach2 = jbu_reach2();
         const int bx = __float2int_rz(ox), by = __float2int_rz(oy);
         const float fx = ox - (float)bx, fy = oy - (float)by;
-        const int nj = min(nn, 7);
+        const int nj = min(nn, reach2 < 49.0f ? 7 : 8);
         for (int j = -nj; j <= nj; ++j) {
             const float dy = fy - (float)j;
             /* the row's taps within reach, and at most one more at each end */
-            const int ni = min(nn, (int)sqrtf(fmaxf(kJbuReach2 - dy * dy, 0.0f)) + 1);
+            const int ni = min(nn, (int)sqrtf(fmaxf(reach2 - dy * dy, 0.0f)) + 1);
             const float4 *crow = coarse + (size_t)(by + j) * s_cols + bx;
             const float *grow = guide + (size_t)(py + j) * cols + px;
 #pragma unroll 4
@@ -127,22 +168,10 @@ __device__ __forceinline__ float4 jbu_pixel(const float *__restrict__ guide, int
                 s.add(__ldg(crow + i), dx * dx + dy * dy, ref_pix, __ldg(grow + i));
             }
         }
+    } else if (taps == kJbuNear) {
+        jbu_window<true>(guide, cols, rows, coarse, s_cols, s_rows, nn, px, py, ox, oy, ref_pix, s);
     } else {
-        for (int j = -nn; j <= nn; ++j) {
-            const int ry = jbu_coarse(oy + (float)j, s_rows);
-            const int rys = min(max(py + j, 0), rows - 1);
-            const float dy = oy - (float)ry;
-            if (taps == kJbuNear && dy * dy > kJbuReach2) continue;
-            const float *grow = guide + (size_t)rys * cols;
-            for (int i = -nn; i <= nn; ++i) {
-                const int rx = jbu_coarse(ox + (float)i, s_cols);
-                const float dx = ox - (float)rx;
-                const float dis = dx * dx + dy * dy;
-                if (taps == kJbuNear && dis > kJbuReach2) continue;
-                const int rxs = min(max(px + i, 0), cols - 1);
-                s.add(__ldg(coarse + (size_t)ry * s_cols + rx), dis, ref_pix, __ldg(grow + rxs));
-            }
-        }
+        jbu_window<false>(guide, cols, rows, coarse, s_cols, s_rows, nn, px, py, ox, oy, ref_pix, s);
     }
     float4 n = make_float4(s.nx / s.nf, s.ny / s.nf, s.nz / s.nf, 0.0f);
     const float inv = rsqrtf(n.x * n.x + n.y * n.y + n.z * n.z);

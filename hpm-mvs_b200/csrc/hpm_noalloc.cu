@@ -45,11 +45,12 @@ __global__ void k_pack_coarse(const float *__restrict__ depth, const float *__re
 
 /* The context path's JBU (hpm::jbu_pixel), writing the normal as 3 floats
  * per pixel as the caller's buffers hold it. */
+template <bool CUT>
 __global__ void k_jbu_noalloc(const float *__restrict__ guide, int cols, int rows, const float4 *__restrict__ coarse,
                               int s_cols, int s_rows, int image_scale, float *__restrict__ out_depth,
                               float *__restrict__ out_normal)
 {
-    const hpm::JbuTaps taps = hpm::jbu_block_taps(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
+    const hpm::JbuTaps taps = hpm::jbu_block_taps<CUT>(guide, cols, rows, coarse, s_cols, s_rows, image_scale);
     const int px = blockIdx.x * blockDim.x + threadIdx.x;
     const int py = hpm::jbu_block_row() + threadIdx.y;
     if (px >= cols || py >= rows) return;
@@ -117,7 +118,8 @@ extern "C" int hpm_jbu_noalloc(int device, const float *guide, int cols, int row
         void *args[] = {(void *)&guide,  (void *)&cols,   (void *)&rows,           (void *)&coarse,
                         (void *)&s_cols, (void *)&s_rows, (void *)&image_scale_arg, (void *)&out_depth,
                         (void *)&out_normal};
-        if (cudaLaunchKernel((const void *)k_jbu_noalloc, hpm::jbu_grid(cols, rows), block, args, 0, s) != cudaSuccess)
+        auto *kernel = hpm::jbu_cuts(image_scale) ? k_jbu_noalloc<true> : k_jbu_noalloc<false>;
+        if (cudaLaunchKernel((const void *)kernel, hpm::jbu_grid(cols, rows), block, args, 0, s) != cudaSuccess)
             return HPM_ERR_CUDA;
     }
     return HPM_OK;
