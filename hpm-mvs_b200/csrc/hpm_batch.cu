@@ -143,6 +143,14 @@ int make_plan(hpm_ctx *c, const std::vector<hpm_ctx *> &ctxs, const std::vector<
     for (cudaEvent_t &e : pl.join) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "batch events");
     return HPM_OK;
 }
+/* The pixels of a batched pass's half-steps, all problems together. */
+long long batch_pixels(const std::vector<hpm_ctx *> &ctxs)
+{
+    long long pixels = 0;
+    for (const hpm_ctx *b : ctxs) pixels += (long long)b->cams[0].width * rows_covered(b->cams[0].height);
+    return pixels;
+}
+
 /* One batched pass with per-problem parameters and `half_steps` half-steps
  * (the reference's 6 unless the prior-net forms ask for fewer iterations).
  * Each problem's chain goes to its own context's stream, forked from and
@@ -155,9 +163,11 @@ int batch_pass(hpm_ctx *c, Plan &pl, const std::vector<HpmParams> &params, int h
     cudaStream_t s = c->stream;
     const size_t n = pl.ctxs.size();
     std::vector<PMArgs> args(n);
+    const long long pixels = batch_pixels(pl.ctxs);
     for (size_t i = 0; i < n; ++i) {
         const int r = ctx_pass_args(pl.ctxs[i], &params[i], &args[i]);
         if (r) return ctx_fail(c, r, "batched pass, problem %zu: %s", i, hpm_last_error(pl.ctxs[i]));
+        args[i].beside = pixels - (long long)args[i].W * args[i].rows_cov;
     }
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "graph capture");
@@ -204,11 +214,13 @@ int batch_pass(hpm_ctx *c, Plan &pl, const std::vector<HpmParams> &params, int h
 
 /* The half-step tile width for each problem: per view size the fastest of
  * 4, 8 and 16 pixels per warp row, timed on one half-step of the scene's first
- * problem of that size (its state is re-initialised by the real passes). */
+ * problem of that size, in the block form that the batched pass will use (its
+ * state is re-initialised by the real passes). */
 int tune_tiles(hpm_ctx *c, const std::vector<hpm_ctx *> &ctxs, const std::vector<HpmParams> &params,
                std::vector<int> &ww)
 {
     ww.assign(ctxs.size(), 8);
+    const long long pixels = batch_pixels(ctxs);
     for (size_t i = 0; i < ctxs.size(); ++i) {
         const HpmCamera &cam = ctxs[i]->cams[0];
         const long long key = ((long long)cam.width << 32) | (unsigned)cam.height;
@@ -224,6 +236,7 @@ int tune_tiles(hpm_ctx *c, const std::vector<hpm_ctx *> &ctxs, const std::vector
                 PMArgs a;
                 const int r = ctx_pass_args(ctxs[i], &params[i], &a);
                 if (r) return ctx_fail(c, r, "tile tuning: %s", hpm_last_error(ctxs[i]));
+                a.beside = pixels - (long long)a.W * a.rows_cov;
                 CK(launch_init(a, c->stream), "tuning init");
                 CK(cudaEventRecord(e0, c->stream), "tuning");
                 CK(launch_propagate(a, 0, 0, c->stream, cand), "tuning half-step");

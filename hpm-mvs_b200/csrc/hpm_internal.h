@@ -41,6 +41,7 @@ struct PMArgs {
     int n; /* images */
     int W, H;
     int rows_cov; /* rows reached by the reference's checkerboard grid */
+    long long beside; /* pixels of the passes that run at the same time (batched forms) */
     float dmin, dmax;
     int geom, prior;
     uint32_t seed_lo, seed_hi, salt;

@@ -2093,12 +2093,15 @@ cudaError_t launch_prop_t(const PMArgs &a, int iter, int color, dim3 grid, cudaS
                        : launch_refine<false, WW, false, NW>(a, iter, color, grid, s);
 }
 
-/* Warps per block of 64 pixels.  Two where the grid fills the GPU; on small
+/* Warps per block of 64 pixels.  Two where the blocks fill the GPU; on small
  * images, where a block's chain of windows is all there is to wait for, more
- * warps share them: eight while two such blocks per SM hold the grid (148 SMs),
+ * warps share them: eight while two such blocks per SM hold them (148 SMs),
  * four while four do.  A pass in ms with 2, 4 and 8 warps, by blocks: 54 0.80,
  * 0.58, 0.51; 247 1.85, 1.43, 1.28; 294 1.86, 1.45, 1.30; 345 3.81, 2.96, 3.01;
- * 486 1.29, 1.14, 1.35; 600 2.32, 2.28, 2.39; 950 2.94, 3.62, 4.58. */
+ * 486 1.29, 1.14, 1.35; 600 2.32, 2.28, 2.39; 950 2.94, 3.62, 4.58.  The blocks
+ * of all passes that run at the same time count (a.beside): a batched scene of
+ * 12 views of 160x120 (150 blocks each) takes 32.3 ms with eight warps, as one
+ * view alone would have them, and 24.4 with two. */
 constexpr long long kBlocks8 = 2 * 148, kBlocks4 = 4 * 148;
 template <int SMAX, int WW>
 cudaError_t launch_prop_n(const PMArgs &a, int iter, int color, cudaStream_t s)
@@ -2106,7 +2109,7 @@ cudaError_t launch_prop_n(const PMArgs &a, int iter, int color, cudaStream_t s)
     constexpr int WH = 32 / WW;
     const dim3 grid((a.W + 2 * WW - 1) / (2 * WW), (a.rows_cov + 2 * WH - 1) / (2 * WH));
     if constexpr (WW == 8) {
-        const long long blocks = (long long)grid.x * grid.y;
+        const long long blocks = (long long)grid.x * grid.y + a.beside / (2 * kBlock);
         if (blocks <= kBlocks8) return launch_prop_t<SMAX, WW, 8>(a, iter, color, grid, s);
         if (blocks <= kBlocks4) return launch_prop_t<SMAX, WW, 4>(a, iter, color, grid, s);
     }
