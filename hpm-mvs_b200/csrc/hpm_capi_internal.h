@@ -133,7 +133,7 @@ struct hpm_ctx {
     std::vector<std::pair<long long, int>> tile_ww;
     hpm::FlowWorkspace flow;
     hpm::HostCopier *copier = nullptr; /* pinned buffers of ctx_copy_in / ctx_copy_out */
-    size_t staged_so_far = 0;          /* bytes that could have used them, while there are none */
+    size_t staged_so_far = 0;          /* bytes in that could have used them, while there are none */
     /* HpmProblemOpts.fix_quirks of the problem being processed (prior levels) */
     bool fix_quirks = false;
     float *d_scene = nullptr; /* hpm_run_scene's per-view maps, grown on demand */

@@ -15,14 +15,12 @@
  * in: 1.8 against 3.1; 38 MB out: 1.5 against 1.9), and so does pinned or
  * device memory, which needs no staging.
  *
- * The pinned buffers themselves take 11 to 25 ms to make, more than a copy of
- * a few tens of MB saves, so a context that lives for one problem goes without
- * them (worth_it).  A new context's first hpm_set_views in ms, with buffers
- * made on the first large copy and now: 20 MB 19.2, 7.0; 38 MB 22.0, 9.0;
- * 40 MB in 21 images 32.0, 18.9; 100 MB 28.4, 18.3; 300 MB 32.1, 32.9 (all
- * plain: 38.0).
+ * The buffers are huge pages of the process, registered with the driver: 16 MB
+ * in 1.2 ms, where cudaHostAlloc takes 10 to 25 and registering small pages 5.
+ * That is still more than one copy of a few tens of MB saves (worth_it).
  */
 #include <string.h>
+#include <sys/mman.h>
 
 #include <atomic>
 #include <exception>
@@ -39,11 +37,13 @@ namespace {
 constexpr size_t kChunk = 1 << 20;
 constexpr int kMaxThreads = 8, kSlots = 2;
 constexpr size_t kMinIn = 16 << 20, kMinOut = 32 << 20;
-constexpr size_t kNowIn = 256 << 20, kNowOut = 128 << 20, kSoFar = 512 << 20;
+constexpr size_t kWorth = 64 << 20;
+constexpr size_t kHugePage = 2 << 20, kPinned = kMaxThreads * kSlots * kChunk;
 }  // namespace
 
 struct HostCopier {
-    char *pinned = nullptr; /* [kMaxThreads][kSlots][kChunk] */
+    void *map = MAP_FAILED; /* kPinned and a huge page, for the alignment */
+    char *pinned = nullptr; /* [kMaxThreads][kSlots][kChunk], once registered */
     cudaEvent_t done[kMaxThreads][kSlots] = {};
 };
 
@@ -56,51 +56,12 @@ void host_copier_free(HostCopier *h)
                 cudaEventSynchronize(e);
                 cudaEventDestroy(e);
             }
-    if (h->pinned) cudaFreeHost(h->pinned);
+    if (h->pinned) cudaHostUnregister(h->pinned);
+    if (h->map != MAP_FAILED) munmap(h->map, kPinned + kHugePage);
     delete h;
 }
 
 namespace {
-
-HostCopier *copier_of(hpm_ctx *c)
-{
-    if (c->copier) return c->copier;
-    HostCopier *h = new (std::nothrow) HostCopier;
-    if (!h) return nullptr;
-    cudaError_t e = cudaHostAlloc((void **)&h->pinned, kMaxThreads * kSlots * kChunk, cudaHostAllocDefault);
-    for (int t = 0; t < kMaxThreads && e == cudaSuccess; ++t)
-        for (int s = 0; s < kSlots && e == cudaSuccess; ++s)
-            e = cudaEventCreateWithFlags(&h->done[t][s], cudaEventDisableTiming);
-    if (e != cudaSuccess) { /* the plain copy needs neither */
-        (void)cudaGetLastError();
-        host_copier_free(h);
-        return nullptr;
-    }
-    c->copier = h;
-    return h;
-}
-
-/* Whether a copy of `bytes` pageable bytes, large enough for the threads, gets
- * pinned buffers to go through where the context has none yet: when this copy
- * alone saves more than they cost, or when the copies that this context has
- * made without them add up to a long-lived one's (bytes out count twice, as
- * they save twice as much). */
-bool worth_it(hpm_ctx *c, size_t bytes, bool out)
-{
-    if (c->copier) return true;
-    c->staged_so_far += out ? 2 * bytes : bytes;
-    return bytes >= (out ? kNowOut : kNowIn) || c->staged_so_far >= kSoFar;
-}
-
-bool pageable(const void *p)
-{
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return at.type == cudaMemoryTypeUnregistered;
-}
 
 /* runs work(thread number) on up to `threads` threads, this one among them */
 template <typename F>
@@ -114,6 +75,59 @@ void on_threads(int threads, F work)
     }
     work(0);
     for (std::thread &t : more) t.join();
+}
+
+HostCopier *copier_of(hpm_ctx *c)
+{
+    if (c->copier) return c->copier;
+    HostCopier *h = new (std::nothrow) HostCopier;
+    if (!h) return nullptr;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    h->map = mmap(nullptr, kPinned + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (h->map != MAP_FAILED) {
+        char *p = (char *)h->map + (kHugePage - (size_t)h->map % kHugePage) % kHugePage;
+        /* without huge pages it only takes longer; a child of this process
+         * must not share pages that transfers write to */
+        (void)madvise(p, kPinned, MADV_HUGEPAGE);
+        (void)madvise(p, kPinned, MADV_DONTFORK);
+        on_threads(kMaxThreads, [p](int t) { /* a huge page's zeroing per thread */
+            for (size_t at = t * (kPinned / kMaxThreads); at < (t + 1) * (kPinned / kMaxThreads); at += kHugePage)
+                *(volatile char *)(p + at) = 0;
+        });
+        e = cudaHostRegister(p, kPinned, cudaHostRegisterDefault);
+        if (e == cudaSuccess) h->pinned = p;
+    }
+    for (int t = 0; t < kMaxThreads && e == cudaSuccess; ++t)
+        for (int s = 0; s < kSlots && e == cudaSuccess; ++s)
+            e = cudaEventCreateWithFlags(&h->done[t][s], cudaEventDisableTiming);
+    if (e != cudaSuccess) { /* the plain copy needs neither */
+        (void)cudaGetLastError();
+        host_copier_free(h);
+        return nullptr;
+    }
+    c->copier = h;
+    return h;
+}
+
+/* Whether a copy of `bytes` pageable bytes, large enough for the threads, gets
+ * pinned buffers to go through where the context has none yet: out of the
+ * device it saves more than they cost; into it only a larger one does, or the
+ * context's copies so far together. */
+bool worth_it(hpm_ctx *c, size_t bytes, bool out)
+{
+    if (c->copier || out) return true;
+    c->staged_so_far += bytes;
+    return c->staged_so_far >= kWorth;
+}
+
+bool pageable(const void *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeUnregistered;
 }
 
 cudaError_t copy(hpm_ctx *c, const CopyItem *items, int n, bool out)
