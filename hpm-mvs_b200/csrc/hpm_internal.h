@@ -59,11 +59,14 @@ struct PMArgs {
     const float4 *prior_planes;
     const uint32_t *masks;
     float *cost_cache; /* [S][colour][ceil(H*W/2)] cost vector of the current hypothesis, or nullptr */
-    /* hand-off between the two kernels of a half-step (L2-resident):
+    /* hand-off between the three kernels of a half-step (L2-resident):
      * cand_costs [kCandRows*S][ceil(H*W/2)] cost matrix rows (8 NESP
      * directions, the refinement candidates and the proposal), cand_pos
-     * [8][ceil(H*W/2)] chosen sites, cand_flags [ceil(H*W/2)] row codes;
-     * indexed by (y * W + x) >> 1, dense over the pixels of one colour */
+     * [8][ceil(H*W/2)] chosen sites, cand_flags [ceil(H*W/2)]: from the
+     * directions to the selection the code of each direction's row, from the
+     * selection to the refinement the row of the chosen plane's costs and
+     * (16) whether the selected views change; indexed by (y * W + x) >> 1,
+     * dense over the pixels of one colour */
     float *cand_costs;
     int *cand_pos;
     uint32_t *cand_flags;

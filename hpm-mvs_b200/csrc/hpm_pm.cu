@@ -47,8 +47,9 @@ constexpr int kBlock = kBlockX * kBlockY;
  * over 32 / ww rows, so that the 32 lanes sample a compact 2D patch of each
  * source image (the texture cache is tiled in 2D).  A block is two such
  * warps stacked vertically.  ww is 8 unless the batched form's tile tuning
- * picks 4 or 16 for a view size. */
-static_assert(kBlock == 64, "two warps per block");
+ * picks 4 or 16 for a view size; wide blocks have further warps, which own no
+ * pixels (launch_prop_n). */
+static_assert(kBlock == 64, "two warps own a block's pixels");
 
 /* (px, py) of this thread in a half-step of `color`, for the block's tile
  * (bx, by) */
@@ -60,11 +61,11 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
 }
 
 /* Blocks per SM that the window kernels are compiled for: 14 to 16 warps, so
- * that nothing spills and the blocks' shared memory leaves 92 KB or more to
- * the texture cache (1600x1200, 5 sources, at 7, 8, 9 and 10 blocks:
- * k_prop_dirs 1.70, 1.68, 1.71, 1.73 ms, k_prop_refine 0.95, 0.96, 2.14, 2.13;
- * 641x481 with 4 sources behaves alike; k_init with 10 sources at 6, 8 and 10
- * blocks: 1.05, 1.02, 1.67 ms). */
+ * that no more than a few words of a thread spill and the blocks' shared memory
+ * leaves 92 KB or more to the texture cache (1600x1200, 5 sources, at 7, 8, 9 and
+ * 10 blocks: k_prop_dirs 1.70, 1.68, 1.71, 1.73 ms, k_prop_refine 0.95, 0.96,
+ * 2.14, 2.13; 641x481 with 4 sources behaves alike; k_init with 10 sources at 6, 8
+ * and 10 blocks: 1.05, 1.02, 1.67 ms). */
 #ifndef HPM_P0_MIN_BLOCKS
 #define HPM_P0_MIN_BLOCKS 8
 #endif
@@ -74,11 +75,12 @@ __device__ __forceinline__ void half_step_pixel_at(int bx, int by, int ww, int c
 #ifndef HPM_P2_MIN_BLOCKS
 #define HPM_P2_MIN_BLOCKS 7
 #endif
+/* warps per SM of their wide forms for small images (kBlocks8) */
+constexpr int kWideWarps = 16;
 /* k_prop_select waits for loads (cost rows, source depths): 32 warps, although
  * some registers spill (1600x1200, 10 sources, plain and geometric pass, by
- * blocks per SM: 6 0.76 and 0.83 ms, 12 0.50 and 0.83, 16 0.47 and 0.71). */
-/* and of their wide forms for small images (kBlocks8) */
-constexpr int kWideWarps = 16;
+ * blocks per SM: 6 0.76 and 0.83 ms, 12 0.50 and 0.83, 16 0.47 and 0.71; with
+ * rows loaded a view ahead, which came later, 0.28 in a plain pass at 16). */
 #ifndef HPM_P3_MIN_BLOCKS
 #define HPM_P3_MIN_BLOCKS 16
 #endif
@@ -1911,7 +1913,7 @@ __device__ __forceinline__ void ends(float *x)
     for (int i = K / 2; i < K - 1; ++i) order(x[i], x[K - 1]);
 }
 
-/* The median of 21 values by forgetting: of any 12 of them neither the least
+/* The median of 21 values by forgetful selection: of any 12 of them neither the least
  * nor the greatest can be the median, so both are dropped and the next value
  * comes in, until three are left.  x is used up. */
 template <int K = 12>
@@ -1928,8 +1930,9 @@ __device__ __forceinline__ float median21(float *x, const float *rest)
 
 /* CheckerboardFilter, HPM.cu:1766-1904.  Away from the borders all 21 depths
  * are there and the median is taken in registers; sorting them in a local
- * array was all of the kernel's time (1600x1200, one colour: 173 us, now 43).  At the borders, and where a depth is not a number (the sort's
- * order then matters), the reference's sort runs. */
+ * array was all of the kernel's time (1600x1200, one colour: 173 us, now 43).
+ * At the borders, and where a depth is not a number (the sort's order then
+ * matters), the reference's sort runs. */
 __global__ void k_filter(const __grid_constant__ PMArgs a, float4 *pl, const float *costs, int color)
 {
     const int py = blockIdx.y * blockDim.y + threadIdx.y;
@@ -2034,7 +2037,7 @@ __global__ void k_geom_costs(const __grid_constant__ PMArgs a, const float4 *pla
 }
 
 /* The 36 source samples of the NCC window of listed pixels, per source view
- * (the values ncc() weighs), and whether the warped centre is inside. */
+ * (the values ncc_quad weighs), and whether the warped centre is inside. */
 __global__ void k_tap_samples(const __grid_constant__ PMArgs a, const float4 *planes, const int *pixels, int n,
                               float *out, int *inside)
 {
